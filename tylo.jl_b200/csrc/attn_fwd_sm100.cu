@@ -74,7 +74,7 @@ template <int DB> struct FwdSmem {
                        O_READY = P_FULL + 2, Q_EMPTY = O_READY + 2, O_FREE = Q_EMPTY + 1, DONE = O_FREE + 2,
                        kNumBars = DONE + 1;
   // Q_EMPTY: every Q K^T product of the finished work item has been issued, its Q tiles may be overwritten;
-  // O_FREE: the softmax warpgroup has read the item's accumulator out of tensor memory.
+  // O_FREE: the softmax warpgroup has read the item's accumulator out of tensor memory (items in which its tile has keys).
   static constexpr int kMisc = kBars + 8 * kNumBars;    // tmem base, abort flag
   static constexpr int kItems = kMisc + 16;             // item table
   static constexpr int kStage = (kItems + kMaxItems * IT_WORDS * 4 + 1023) / 1024 * 1024;   // 8 softmax warps x 2 KB of output staging
@@ -832,7 +832,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           volatile int* w = e + X * WI_WORDS;
           w[WI_B] = it.b; w[WI_H] = it.h + X * plan.h_step; w[WI_Q0] = it.q0 + X * plan.q_step; w[WI_KLEN] = it.k_len;
           w[WI_QLIM] = it.q_lim; w[WI_KV0] = (it.jlo + it.tr[X].s) * BN; w[WI_N] = it.tr[X].e - it.tr[X].s;
-          w[WI_RELEASE] = it.n_tot > 0;
+          w[WI_RELEASE] = it.tr[X].e > it.tr[X].s;
         }
         e[IT_NTOT] = it.n_tot; e[IT_JLO] = it.jlo; e[IT_AS] = it.tr[0].s; e[IT_AE] = it.tr[0].e; e[IT_BS] = it.tr[1].s;
         e[IT_BE] = it.tr[1].e; e[IT_HK] = it.hk; e[IT_HEAD] = it.h; e[IT_Q0] = it.q0; e[IT_BATCH] = it.b;
@@ -917,6 +917,8 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         bool ok = true;
         int ni = 0, g0 = 0;      // non-empty items and K/V tiles of the items before this one
         int cb[2] = {0, 0};      // key tiles each Q tile took part in before this item (S / P / O phases)
+        int na[2] = {0, 0};      // items before this one in which each Q tile had keys (O_FREE phases: a warpgroup without
+                                 // keys does not arrive, or it could run two phases ahead of the wait below)
         for (int k = 0; k < n_local && ok; ++k) {
           volatile int* e = tab + k * IT_WORDS;
           const int n_tot = e[IT_NTOT];
@@ -961,8 +963,8 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
               if (active(X, j)) {
                 if (!v_ready) { ok = mbar_wait(bar(SM::V_FULL + st), (gj / ST) & 1, abort_flag, &g_attn_fwd_status, 204); v_ready = true; }
                 // the accumulator of the item before must have been read out before it is overwritten
-                if (j == ts[X] && ni > 0)
-                  ok = ok && mbar_wait(bar(SM::O_FREE + X), (ni - 1) & 1, abort_flag, &g_attn_fwd_status, 206);
+                if (j == ts[X] && na[X] > 0)
+                  ok = ok && mbar_wait(bar(SM::O_FREE + X), (na[X] - 1) & 1, abort_flag, &g_attn_fwd_status, 206);
                 ok = ok && mbar_wait(bar(SM::P_FULL + X), (cb[X] + j - ts[X]) & 1, abort_flag, &g_attn_fwd_status, 205);
                 if (!ok) break;
                 tc_fence_after();
@@ -985,11 +987,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
               if (j + 2 == n_tot) tc_commit(bar(SM::Q_EMPTY));   // every Q K^T product of the item is issued
             }
           }
-          // a Q tile without keys in this item: keep in step with its warpgroup's O_FREE phases
-#pragma unroll
-          for (int X = 0; X < 2; ++X)
-            if (ok && ni > 0 && te[X] == ts[X])
-              ok = mbar_wait(bar(SM::O_FREE + X), (ni - 1) & 1, abort_flag, &g_attn_fwd_status, 207);
+          na[0] += te[0] > ts[0]; na[1] += te[1] > ts[1];
           cb[0] += te[0] - ts[0]; cb[1] += te[1] - ts[1];
           g0 += n_tot; ++ni;
         }
