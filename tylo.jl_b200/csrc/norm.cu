@@ -18,12 +18,14 @@ namespace tylo {
 
 #define TYLO_ROW_DISPATCH(shape, ...)                                                          \
   do {                                                                                         \
-    if ((shape).threads == 32 && (shape).iters == 2) { constexpr int THREADS = 32, ITERS = 2; __VA_ARGS__; }          \
+    if ((shape).threads == 32) { constexpr int THREADS = 32, ITERS = 2; __VA_ARGS__; }                                \
+    else if ((shape).threads == 64) { constexpr int THREADS = 64, ITERS = 2; __VA_ARGS__; }                           \
     else if ((shape).threads == 128 && (shape).iters == 2) { constexpr int THREADS = 128, ITERS = 2; __VA_ARGS__; }   \
-    else if ((shape).threads == 256 && (shape).iters == 4) { constexpr int THREADS = 256, ITERS = 4; __VA_ARGS__; }   \
-    else if ((shape).threads == 512 && (shape).iters == 8) { constexpr int THREADS = 512, ITERS = 8; __VA_ARGS__; }   \
-    else if ((shape).threads == 1024 && (shape).iters == 8) { constexpr int THREADS = 1024, ITERS = 8; __VA_ARGS__; } \
-    else { constexpr int THREADS = 1024, ITERS = 4; __VA_ARGS__; }                                                    \
+    else if ((shape).threads == 128) { constexpr int THREADS = 128, ITERS = 4; __VA_ARGS__; }                         \
+    else if ((shape).threads == 256) { constexpr int THREADS = 256, ITERS = 4; __VA_ARGS__; }                         \
+    else if ((shape).threads == 512 && (shape).iters == 4) { constexpr int THREADS = 512, ITERS = 4; __VA_ARGS__; }   \
+    else if ((shape).threads == 512) { constexpr int THREADS = 512, ITERS = 8; __VA_ARGS__; }                         \
+    else { constexpr int THREADS = 1024, ITERS = 8; __VA_ARGS__; }                                                    \
   } while (0)
 
 // Merge of two (count, mean, M2) partial statistics.
@@ -99,15 +101,16 @@ __device__ __forceinline__ void welford_block(float& n, float& mu, float& m2, fl
 // forward, row in registers
 // ------------------------------------------------------------------------------------------------
 template <typename T, int THREADS, int ITERS, bool LAYER>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(row_cta(THREADS))
 norm_fwd_kernel(T* __restrict__ Y, const T* __restrict__ X, const T* __restrict__ W,
                 const T* __restrict__ Bias, float* __restrict__ Mean, float* __restrict__ Rstd,
-                int M, float eps, float offset) {
+                int M, int N, float eps, float offset) {
   constexpr int VEC = Elem<T>::kVec;
   __shared__ float red[32];
   __shared__ float wred[LAYER ? 96 : 1];
-  const int nvec = M / VEC;
-  const size_t row = blockIdx.x;
+  const int nvec = M / VEC, tid = row_thread<THREADS>();
+  const size_t row = row_index<THREADS>();
+  if (THREADS == 32 && row >= (size_t)N) return;
   RowRegs<T, THREADS, ITERS> x;
   x.load(X + row * M, nvec);
 
@@ -123,7 +126,7 @@ norm_fwd_kernel(T* __restrict__ Y, const T* __restrict__ X, const T* __restrict_
     uint64_t s2 = 0ull;
 #pragma unroll
     for (int i = 0; i < ITERS; ++i) {
-      if (i * THREADS + (int)threadIdx.x < nvec) {
+      if (i * THREADS + tid < nvec) {
         float f[VEC]; x.p[i].unpack(f);
 #pragma unroll
         for (int j = 0; j < VEC; j += 2) s2 = sm100::add_f32x2(s2, sm100::pack_f32x2(f[j], f[j + 1]));
@@ -136,7 +139,7 @@ norm_fwd_kernel(T* __restrict__ Y, const T* __restrict__ X, const T* __restrict_
     uint64_t q2 = 0ull;
 #pragma unroll
     for (int i = 0; i < ITERS; ++i) {
-      if (i * THREADS + (int)threadIdx.x < nvec) {
+      if (i * THREADS + tid < nvec) {
         float f[VEC]; x.p[i].unpack(f);
 #pragma unroll
         for (int j = 0; j < VEC; j += 2) {
@@ -164,13 +167,13 @@ norm_fwd_kernel(T* __restrict__ Y, const T* __restrict__ X, const T* __restrict_
     ss = block_reduce<THREADS>(ss, SumOp(), 0.f, red);
   }
   const float rstd = 1.0f / sqrtf(ss * inv_m + eps);
-  if (threadIdx.x == 0) {
+  if (tid == 0) {
     if (Rstd) Rstd[row] = rstd;
     if (LAYER && Mean) Mean[row] = mean;
   }
 #pragma unroll
   for (int i = 0; i < ITERS; ++i) {
-    const int v = i * THREADS + threadIdx.x;
+    const int v = i * THREADS + tid;
     if (v < nvec) {
       float f[VEC], w[VEC], b[VEC];
       x.p[i].unpack(f);
@@ -238,101 +241,6 @@ norm_fwd_generic_kernel(T* __restrict__ Y, const T* __restrict__ X, const T* __r
 // ------------------------------------------------------------------------------------------------
 // backward
 // ------------------------------------------------------------------------------------------------
-template <typename T, int THREADS, int ITERS, bool LAYER>
-__global__ void __launch_bounds__(THREADS)
-norm_bwd_kernel(T* __restrict__ dX, float* __restrict__ dWp, float* __restrict__ dBp,
-                const T* __restrict__ dY, const T* __restrict__ X, const T* __restrict__ W,
-                const float* __restrict__ Mean, const float* __restrict__ Rstd,
-                int M, int64_t N, float offset) {
-  constexpr int VEC = Elem<T>::kVec;
-  __shared__ float red[64];
-  const int nvec = M / VEC;
-  const float inv_m = 1.0f / (float)M;
-
-  float g[ITERS][VEC];       // w (+offset) for the columns this thread owns
-  float dw[ITERS][VEC], db[LAYER ? ITERS : 1][VEC];
-#pragma unroll
-  for (int i = 0; i < ITERS; ++i) {
-    const int v = i * THREADS + threadIdx.x;
-    if (v < nvec) ld_param(W + (size_t)v * VEC).unpack(g[i]);
-#pragma unroll
-    for (int j = 0; j < VEC; ++j) {
-      if (v >= nvec) g[i][j] = 0.f;
-      if constexpr (!LAYER) g[i][j] += offset;
-      dw[i][j] = 0.f;
-      if constexpr (LAYER) db[i][j] = 0.f;
-    }
-  }
-
-  for (int64_t row = blockIdx.x; row < N; row += gridDim.x) {
-    RowRegs<T, THREADS, ITERS> x, dy;
-    x.load(X + row * M, nvec);
-    dy.load(dY + row * M, nvec);
-    const float rstd = Rstd[row];
-    const float mean = LAYER ? Mean[row] : 0.f;
-    // c1 = mean(xhat * g*dy), c2 = mean(g*dy) (LayerNorm only)
-    float s1 = 0.f, s2 = 0.f;
-#pragma unroll
-    for (int i = 0; i < ITERS; ++i) {
-      float xf[VEC], df[VEC];
-      x.p[i].unpack(xf); dy.p[i].unpack(df);
-#pragma unroll
-      for (int j = 0; j < VEC; ++j) {
-        const float xhat = (xf[j] - mean) * rstd;   // zero packets contribute g = 0
-        const float gd = g[i][j] * df[j];
-        s1 += xhat * gd;
-        if constexpr (LAYER) s2 += gd;
-      }
-    }
-    // two sums through one reduction round
-    s1 = warp_reduce(s1, SumOp());
-    if constexpr (LAYER) s2 = warp_reduce(s2, SumOp());
-    if constexpr (THREADS > 32) {
-      const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-      if (lane == 0) { red[warp] = s1; red[32 + warp] = s2; }
-      __syncthreads();
-      float a = lane < THREADS / 32 ? red[lane] : 0.f;
-      float b = lane < THREADS / 32 ? red[32 + lane] : 0.f;
-      s1 = warp_reduce(a, SumOp());
-      if constexpr (LAYER) s2 = warp_reduce(b, SumOp());
-      __syncthreads();
-    }
-    const float c1 = s1 * inv_m, c2 = s2 * inv_m;
-#pragma unroll
-    for (int i = 0; i < ITERS; ++i) {
-      float xf[VEC], df[VEC], o[VEC];
-      x.p[i].unpack(xf); dy.p[i].unpack(df);
-#pragma unroll
-      for (int j = 0; j < VEC; ++j) {
-        const float xhat = (xf[j] - mean) * rstd;
-        const float gd = g[i][j] * df[j];
-        // RMS: rstd*(dy*g - rstd^2*dd*x) with xhat = x*rstd, c1 = rstd*dd  (test/norm.jl:78-87)
-        // LN : (g*dy - (xhat*c1 + c2))*rstd                                  (test/norm.jl:90-102)
-        o[j] = (gd - (xhat * c1 + c2)) * rstd;
-        dw[i][j] += df[j] * xhat;
-        if constexpr (LAYER) db[i][j] += df[j];
-      }
-      x.p[i].pack(o);
-    }
-    x.store(dX + row * M, nvec);
-  }
-
-#pragma unroll
-  for (int i = 0; i < ITERS; ++i) {
-    const int v = i * THREADS + threadIdx.x;
-    if (v < nvec) {
-      float4* pw = reinterpret_cast<float4*>(dWp + (size_t)blockIdx.x * M + (size_t)v * VEC);
-#pragma unroll
-      for (int j = 0; j < VEC; j += 4) pw[j / 4] = make_float4(dw[i][j], dw[i][j + 1], dw[i][j + 2], dw[i][j + 3]);
-      if constexpr (LAYER) {
-        float4* pb = reinterpret_cast<float4*>(dBp + (size_t)blockIdx.x * M + (size_t)v * VEC);
-#pragma unroll
-        for (int j = 0; j < VEC; j += 4) pb[j / 4] = make_float4(db[i][j], db[i][j + 1], db[i][j + 2], db[i][j + 3]);
-      }
-    }
-  }
-}
-
 // backward, streaming form for rows of exactly THREADS packets (one 16-byte packet of X and of dY per
 // thread): the per-thread state is a handful of registers, so the packets of the next TWO rows are
 // already in flight while the current row is reduced — the HBM stream never waits for a reduction.
@@ -434,81 +342,340 @@ norm_bwd_stream_kernel(T* __restrict__ dX, float* __restrict__ dWp, float* __res
   }
 }
 
-// backward for any M / alignment: the CTA's partial row is accumulated in global memory
-// (the CTA is its only writer).
-template <typename T, bool LAYER>
-__global__ void __launch_bounds__(256)
+// Rows of up to 1,024 packets: one 16-byte packet of X and dY per thread, TPR threads (whole warps) per row, R rows per CTA at
+// a time.  HBM bound; what it takes is bytes in flight, so short rows share a CTA (a 512-element bf16 row is 64 threads:
+// alone in its CTA it left 2 warps per SM, 8 rows give 32) and every row group asks for its next one or two rows before it
+// reduces the current one, so that the stream never waits for a reduction.  One named barrier per row (scratch is
+// double-buffered); none when a row is one warp.  dW / dB partials stay in registers and are added up over the R groups
+// through shared memory at the end.
+constexpr int kMaxSmem = 220 * 1024;    // dynamic shared memory asked for at most
+constexpr int kNormRowGroups = 15;      // named barriers 1..15
+
+template <typename T, bool LAYER, bool FULL>      // FULL: every thread of a row holds a packet
+__global__ void __launch_bounds__(1024)
+norm_bwd_kernel(T* __restrict__ dX, float* __restrict__ dWp, float* __restrict__ dBp, const T* __restrict__ dY,
+                const T* __restrict__ X, const T* __restrict__ W, const float* __restrict__ Mean,
+                const float* __restrict__ Rstd, int M, int N, float offset, int tpr, int R) {
+  constexpr int VEC = Elem<T>::kVec;
+  extern __shared__ __align__(16) float sm[];
+  const int nvec = FULL ? tpr : M / VEC, wpr = tpr >> 5;
+  const int rg = threadIdx.x / tpr, v = threadIdx.x % tpr, lane = threadIdx.x & 31, wr = v >> 5;
+  float* red = sm + rg * 2 * 64;               // [parity][64]
+  float* tot = sm + R * 2 * 64;                // the CTA's dW (and dB) partials, R > 1
+  const bool live = FULL || v < nvec;
+  const int col = v * VEC;
+  const float inv_m = 1.0f / (float)M;
+  float g[VEC], dw[VEC], db[VEC];
+  if (live) ld_param(W + col).unpack(g);
+#pragma unroll
+  for (int j = 0; j < VEC; ++j) {
+    g[j] = live ? (LAYER ? g[j] : g[j] + offset) : 0.f;
+    dw[j] = 0.f; db[j] = 0.f;
+  }
+  const int stride = (int)gridDim.x * R;        // (at most 296 x 15, see the launch)
+  Pack<T> x0, d0, x1, d1, x2, d2;
+  x0.raw = d0.raw = x1.raw = d1.raw = x2.raw = d2.raw = make_uint4(0, 0, 0, 0);
+  float r0 = 0.f, r1 = 0.f, r2 = 0.f, m0 = 0.f, m1 = 0.f, m2 = 0.f;
+  auto fetch = [&](int r, Pack<T>& x, Pack<T>& d, float& rs, float& mn) {
+    if ((unsigned)r < (unsigned)N) {
+      if (live) { x.raw = ld_stream(X + (size_t)r * M + col); d.raw = ld_stream(dY + (size_t)r * M + col); }
+      rs = Rstd[r];
+      mn = LAYER ? Mean[r] : 0.f;
+    }
+  };
+  // rows in flight behind the current one: two for RMSNorm, one for LayerNorm (its extra accumulators
+  // and statistics would otherwise push the 1024-thread CTA past 64 registers per thread)
+  int row = (int)blockIdx.x * R + rg;
+  fetch(row, x0, d0, r0, m0);
+  if constexpr (!LAYER) fetch(row + stride, x1, d1, r1, m1);
+  for (int par = 0; (unsigned)row < (unsigned)N; row += stride, par ^= 1) {
+    if constexpr (LAYER) fetch(row + stride, x1, d1, r1, m1);
+    else fetch(row + 2 * stride, x2, d2, r2, m2);
+    float s1 = 0.f, s2 = 0.f;
+    const uint64_t nm2 = sm100::pack_f32x2(-m0, -m0), r2p = sm100::pack_f32x2(r0, r0);
+    {
+      // packed fp32 pairs: xhat = (x - mean) rstd, gd = g dy, s1 += xhat gd, s2 += gd  (dead lanes have g = 0)
+      float xf[VEC], df[VEC];
+      x0.unpack(xf); d0.unpack(df);
+      uint64_t a1 = 0ull, a2 = 0ull;
+#pragma unroll
+      for (int j = 0; j < VEC; j += 2) {
+        const uint64_t gd2 = sm100::mul_f32x2(sm100::pack_f32x2(g[j], g[j + 1]), sm100::pack_f32x2(df[j], df[j + 1]));
+        const uint64_t xh2 = sm100::mul_f32x2(sm100::add_f32x2(sm100::pack_f32x2(xf[j], xf[j + 1]), nm2), r2p);
+        a1 = sm100::fma_f32x2(xh2, gd2, a1);
+        if constexpr (LAYER) a2 = sm100::add_f32x2(a2, gd2);
+      }
+      float lo, hi;
+      sm100::unpack_f32x2(a1, lo, hi); s1 = lo + hi;
+      if constexpr (LAYER) { sm100::unpack_f32x2(a2, lo, hi); s2 = lo + hi; }
+    }
+    s1 = warp_reduce(s1, SumOp());
+    if constexpr (LAYER) s2 = warp_reduce(s2, SumOp());
+    if (wpr > 1) {
+      float* rp = red + par * 64;
+      if (lane == 0) { rp[wr] = s1; rp[32 + wr] = s2; }
+      asm volatile("bar.sync %0, %1;" ::"r"(rg + 1), "r"(tpr) : "memory");
+      s1 = warp_reduce(lane < wpr ? rp[lane] : 0.f, SumOp());
+      if constexpr (LAYER) s2 = warp_reduce(lane < wpr ? rp[32 + lane] : 0.f, SumOp());
+    }
+    const float c1 = s1 * inv_m, c2 = LAYER ? s2 * inv_m : 0.f;
+    // the packets are unpacked again rather than kept as fp32 across the barrier (registers)
+    float xf[VEC], df[VEC], o[VEC];
+    x0.unpack(xf); d0.unpack(df);
+    const uint64_t nc1 = sm100::pack_f32x2(-c1, -c1), nc2 = sm100::pack_f32x2(-c2, -c2);
+#pragma unroll
+    for (int j = 0; j < VEC; j += 2) {
+      // RMS: rstd*(dy*g - rstd^2*dd*x) with xhat = x*rstd, c1 = rstd*dd  (test/norm.jl:78-87)
+      // LN : (g*dy - (xhat*c1 + c2))*rstd                                  (test/norm.jl:90-102)
+      // two columns per instruction; dW += dy xhat,  dB += dy
+      const uint64_t df2 = sm100::pack_f32x2(df[j], df[j + 1]);
+      const uint64_t xh2 = sm100::mul_f32x2(sm100::add_f32x2(sm100::pack_f32x2(xf[j], xf[j + 1]), nm2), r2p);
+      const uint64_t t2 = sm100::fma_f32x2(xh2, nc1, nc2);
+      const uint64_t o2 = sm100::mul_f32x2(sm100::fma_f32x2(sm100::pack_f32x2(g[j], g[j + 1]), df2, t2), r2p);
+      sm100::unpack_f32x2(o2, o[j], o[j + 1]);
+      const uint64_t w2 = sm100::fma_f32x2(df2, xh2, sm100::pack_f32x2(dw[j], dw[j + 1]));
+      sm100::unpack_f32x2(w2, dw[j], dw[j + 1]);
+      if constexpr (LAYER) {
+        const uint64_t b2 = sm100::add_f32x2(sm100::pack_f32x2(db[j], db[j + 1]), df2);
+        sm100::unpack_f32x2(b2, db[j], db[j + 1]);
+      }
+    }
+    Pack<T> out; out.pack(o);
+    if (live) st_stream(dX + (size_t)row * M + col, out.raw);
+    x0 = x1; d0 = d1; r0 = r1; m0 = m1;
+    if constexpr (!LAYER) { x1 = x2; d1 = d2; r1 = r2; m1 = m2; }
+  }
+  // sum over the row groups, in their order
+  for (int k = 1; k < R; ++k) {
+    if (rg == k && live) {
+#pragma unroll
+      for (int j = 0; j < VEC; ++j) { tot[col + j] = dw[j]; if constexpr (LAYER) tot[M + col + j] = db[j]; }
+    }
+    __syncthreads();
+    if (rg == 0 && live) {
+#pragma unroll
+      for (int j = 0; j < VEC; ++j) { dw[j] += tot[col + j]; if constexpr (LAYER) db[j] += tot[M + col + j]; }
+    }
+    __syncthreads();
+  }
+  if (rg == 0 && live) {
+    float4* pw = reinterpret_cast<float4*>(dWp + (size_t)blockIdx.x * M + col);
+#pragma unroll
+    for (int j = 0; j < VEC; j += 4) pw[j / 4] = make_float4(dw[j], dw[j + 1], dw[j + 2], dw[j + 3]);
+    if constexpr (LAYER) {
+      float4* pb = reinterpret_cast<float4*>(dBp + (size_t)blockIdx.x * M + col);
+#pragma unroll
+      for (int j = 0; j < VEC; j += 4) pb[j / 4] = make_float4(db[j], db[j + 1], db[j + 2], db[j + 3]);
+    }
+  }
+}
+
+// Longer rows (up to 4,096 packets, as long as the accumulators fit shared memory): P packets per thread, one row per CTA at
+// a time, dW / dB partials in shared memory (each thread is the only one to touch its columns), the weights re-read from
+// the first-level cache.
+template <typename T, int P, bool LAYER>
+__global__ void __launch_bounds__(1024)
+norm_bwd_wide_kernel(T* __restrict__ dX, float* __restrict__ dWp, float* __restrict__ dBp, const T* __restrict__ dY,
+                     const T* __restrict__ X, const T* __restrict__ W, const float* __restrict__ Mean,
+                     const float* __restrict__ Rstd, int M, int64_t N, float offset) {
+  constexpr int VEC = Elem<T>::kVec;
+  extern __shared__ __align__(16) float sm[];
+  const int nvec = M / VEC, nt = blockDim.x, wpr = nt >> 5, lane = threadIdx.x & 31, wr = threadIdx.x >> 5;
+  float* red = sm;
+  float* aw = sm + 128;
+  float* ab = aw + M;
+  const float inv_m = 1.0f / (float)M;
+  for (int i = threadIdx.x; i < (LAYER ? 2 : 1) * M; i += nt) aw[i] = 0.f;
+  __syncthreads();
+  int par = 0;
+  for (int64_t row = blockIdx.x; row < N; row += gridDim.x, par ^= 1) {
+    Pack<T> x[P], d[P];
+#pragma unroll
+    for (int i = 0; i < P; ++i) {
+      const int v = i * nt + threadIdx.x;
+      x[i].raw = d[i].raw = make_uint4(0, 0, 0, 0);
+      if (v < nvec) { x[i].raw = ld_stream(X + row * M + (size_t)v * VEC); d[i].raw = ld_stream(dY + row * M + (size_t)v * VEC); }
+    }
+    const float rstd = Rstd[row], mean = LAYER ? Mean[row] : 0.f;
+    float s1 = 0.f, s2 = 0.f;
+#pragma unroll
+    for (int i = 0; i < P; ++i) {
+      const int v = i * nt + threadIdx.x;
+      if (v < nvec) {
+        float xf[VEC], df[VEC], g[VEC];
+        x[i].unpack(xf); d[i].unpack(df); ld_param(W + (size_t)v * VEC).unpack(g);
+#pragma unroll
+        for (int j = 0; j < VEC; ++j) {
+          const float gd = (LAYER ? g[j] : g[j] + offset) * df[j];
+          s1 += (xf[j] - mean) * rstd * gd;
+          if constexpr (LAYER) s2 += gd;
+        }
+      }
+    }
+    s1 = warp_reduce(s1, SumOp());
+    if constexpr (LAYER) s2 = warp_reduce(s2, SumOp());
+    float* rp = red + par * 64;
+    if (lane == 0) { rp[wr] = s1; rp[32 + wr] = s2; }
+    __syncthreads();
+    s1 = warp_reduce(lane < wpr ? rp[lane] : 0.f, SumOp());
+    if constexpr (LAYER) s2 = warp_reduce(lane < wpr ? rp[32 + lane] : 0.f, SumOp());
+    const float c1 = s1 * inv_m, c2 = LAYER ? s2 * inv_m : 0.f;
+#pragma unroll
+    for (int i = 0; i < P; ++i) {
+      const int v = i * nt + threadIdx.x;
+      if (v < nvec) {
+        float xf[VEC], df[VEC], g[VEC], o[VEC];
+        x[i].unpack(xf); d[i].unpack(df); ld_param(W + (size_t)v * VEC).unpack(g);
+        float4* pw = reinterpret_cast<float4*>(aw + (size_t)v * VEC);
+        float4* pb = reinterpret_cast<float4*>(ab + (size_t)v * VEC);
+#pragma unroll
+        for (int q = 0; q < VEC; q += 4) {
+          float xh[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            xh[e] = (xf[q + e] - mean) * rstd;
+            o[q + e] = ((LAYER ? g[q + e] : g[q + e] + offset) * df[q + e] - (xh[e] * c1 + c2)) * rstd;
+          }
+          float4 w = pw[q / 4];
+          w.x += df[q] * xh[0]; w.y += df[q + 1] * xh[1]; w.z += df[q + 2] * xh[2]; w.w += df[q + 3] * xh[3];
+          pw[q / 4] = w;
+          if constexpr (LAYER) {
+            float4 b = pb[q / 4];
+            b.x += df[q]; b.y += df[q + 1]; b.z += df[q + 2]; b.w += df[q + 3];
+            pb[q / 4] = b;
+          }
+        }
+        Pack<T> out; out.pack(o);
+        st_stream(dX + row * M + (size_t)v * VEC, out.raw);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < P; ++i) {
+    const int v = i * nt + threadIdx.x;
+    if (v < nvec) {
+#pragma unroll
+      for (int q = 0; q < VEC; q += 4) {
+        const size_t c = (size_t)v * VEC + q;
+        *reinterpret_cast<float4*>(dWp + (size_t)blockIdx.x * M + c) = *reinterpret_cast<const float4*>(aw + c);
+        if constexpr (LAYER) *reinterpret_cast<float4*>(dBp + (size_t)blockIdx.x * M + c) = *reinterpret_cast<const float4*>(ab + c);
+      }
+    }
+  }
+}
+
+// Any M / alignment: element accesses.  While the row and the partials fit shared memory (SMEM), X and dY are read from
+// memory once, the row waits in shared memory as fp32 and the partials are added up there; beyond that the CTA's partial row
+// is accumulated in global memory (the CTA is its only writer) and the row read twice.
+template <typename T, bool LAYER, bool SMEM>
+__global__ void __launch_bounds__(512)
 norm_bwd_generic_kernel(T* __restrict__ dX, float* __restrict__ dWp, float* __restrict__ dBp,
                         const T* __restrict__ dY, const T* __restrict__ X,
                         const T* __restrict__ W, const float* __restrict__ Mean,
                         const float* __restrict__ Rstd, int64_t M, int64_t N, float offset) {
-  __shared__ float red[32];
+  constexpr int NT = 512, U = 4;
+  __shared__ float red[64];
+  extern __shared__ __align__(16) float sm[];
   const float inv_m = 1.0f / (float)M;
-  float* mw = dWp + (size_t)blockIdx.x * M;
-  float* mb = LAYER ? dBp + (size_t)blockIdx.x * M : nullptr;
-  for (int64_t i = threadIdx.x; i < M; i += 256) { mw[i] = 0.f; if (LAYER) mb[i] = 0.f; }
+  float* mw = SMEM ? sm : dWp + (size_t)blockIdx.x * M;
+  float* mb = !LAYER ? nullptr : (SMEM ? sm + M : dBp + (size_t)blockIdx.x * M);
+  float* cx = sm + (LAYER ? 2 : 1) * M;        // xhat and dy of the row
+  float* cd = cx + M;
+  for (int64_t i = threadIdx.x; i < M; i += NT) { mw[i] = 0.f; if (LAYER) mb[i] = 0.f; }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int64_t row = blockIdx.x; row < N; row += gridDim.x) {
     const T* x = X + row * M; const T* dy = dY + row * M;
     const float rstd = Rstd[row];
     const float mean = LAYER ? Mean[row] : 0.f;
     float s1 = 0.f, s2 = 0.f;
-    for (int64_t i = threadIdx.x; i < M; i += 256) {
-      const float gi = Elem<T>::to_f(W[i]) + (LAYER ? 0.f : offset);
-      const float gd = gi * Elem<T>::to_f(dy[i]);
-      s1 += (Elem<T>::to_f(x[i]) - mean) * rstd * gd;
-      s2 += gd;
+    for (int64_t i0 = threadIdx.x; i0 < M; i0 += NT * U) {
+      float xv[U], dv[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int64_t i = i0 + u * NT;
+        xv[u] = i < M ? Elem<T>::to_f(x[i]) : mean;
+        dv[u] = i < M ? Elem<T>::to_f(dy[i]) : 0.f;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int64_t i = i0 + u * NT;
+        if (i < M) {
+          const float xh = (xv[u] - mean) * rstd, gd = (Elem<T>::to_f(W[i]) + (LAYER ? 0.f : offset)) * dv[u];
+          s1 += xh * gd;
+          s2 += gd;
+          if (SMEM) { cx[i] = xh; cd[i] = dv[u]; }
+        }
+      }
     }
-    const float c1 = block_reduce<256>(s1, SumOp(), 0.f, red) * inv_m;
-    const float c2 = LAYER ? block_reduce<256>(s2, SumOp(), 0.f, red) * inv_m : 0.f;
-    for (int64_t i = threadIdx.x; i < M; i += 256) {
+    s1 = warp_reduce(s1, SumOp());
+    s2 = warp_reduce(s2, SumOp());
+    if (lane == 0) { red[warp] = s1; red[32 + warp] = s2; }
+    __syncthreads();
+    const float c1 = warp_reduce(lane < NT / 32 ? red[lane] : 0.f, SumOp()) * inv_m;
+    const float c2 = LAYER ? warp_reduce(lane < NT / 32 ? red[32 + lane] : 0.f, SumOp()) * inv_m : 0.f;
+    __syncthreads();
+    for (int64_t i = threadIdx.x; i < M; i += NT) {
       const float gi = Elem<T>::to_f(W[i]) + (LAYER ? 0.f : offset);
-      const float d = Elem<T>::to_f(dy[i]);
-      const float xhat = (Elem<T>::to_f(x[i]) - mean) * rstd;
+      const float d = SMEM ? cd[i] : Elem<T>::to_f(dy[i]);
+      const float xhat = SMEM ? cx[i] : (Elem<T>::to_f(x[i]) - mean) * rstd;
       dX[row * M + i] = Elem<T>::from_f((gi * d - (xhat * c1 + c2)) * rstd);
       mw[i] += d * xhat;
       if (LAYER) mb[i] += d;
     }
   }
+  if (SMEM)
+    for (int64_t i = threadIdx.x; i < M; i += NT) {
+      dWp[(size_t)blockIdx.x * M + i] = mw[i];
+      if (LAYER) dBp[(size_t)blockIdx.x * M + i] = mb[i];
+    }
 }
 
-// second stage: dW[m] = sum over groups of the partial rows.
+// second stage: dW[m] = sum over groups of the partial rows.  32 columns x 32 group lanes per CTA, four rows in flight per
+// lane: at 768 columns only 24 CTAs run, and eight lanes adding 37 rows one after the other took 13 us of waiting.
 template <typename T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(1024)
 norm_bwd_reduce_kernel(T* __restrict__ dW, T* __restrict__ dB, const float* __restrict__ dWp,
                        const float* __restrict__ dBp, int64_t M, int n_groups) {
-  // 32 columns x 8 group-lanes per CTA
-  __shared__ float sw[8][33], sb[8][33];
+  __shared__ float sw[32][33], sb[32][33];
   const int col = threadIdx.x & 31, gl = threadIdx.x >> 5;
   const int64_t m = (int64_t)blockIdx.x * 32 + col;
   float aw = 0.f, ab = 0.f;
   if (m < M) {
-    for (int g = gl; g < n_groups; g += 8) {
+#pragma unroll 4
+    for (int g = gl; g < n_groups; g += 32) {
       aw += dWp[(size_t)g * M + m];
       if (dBp) ab += dBp[(size_t)g * M + m];
     }
   }
   sw[gl][col] = aw; sb[gl][col] = ab;
   __syncthreads();
-  if (gl == 0 && m < M) {
-#pragma unroll
-    for (int k = 1; k < 8; ++k) { aw += sw[k][col]; ab += sb[k][col]; }
-    dW[m] = Elem<T>::from_f(aw);
-    if (dBp) dB[m] = Elem<T>::from_f(ab);
+  // warp gl sums column gl over its 32 lanes
+  const float tw = warp_reduce(sw[col][gl], SumOp()), tb = warp_reduce(sb[col][gl], SumOp());
+  const int64_t mo = (int64_t)blockIdx.x * 32 + gl;
+  if (col == 0 && mo < M) {
+    dW[mo] = Elem<T>::from_f(tw);
+    if (dBp) dB[mo] = Elem<T>::from_f(tb);
   }
 }
 
 // ------------------------------------------------------------------------------------------------
 // host side
 // ------------------------------------------------------------------------------------------------
+// Shared memory beyond 48 KB has to be asked for; below that the call would only cost the host time.
+template <typename K> static int32_t allow_smem(K kern, int64_t bytes) {
+  if (bytes > 48 * 1024) TYLO_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  return TYLO_OK;
+}
+
 template <typename T, bool LAYER>
 static int32_t norm_fwd_launch(void* Y, const void* X, const void* W, const void* Bias, float* Mean,
                                float* Rstd, int64_t M, int64_t N, float eps, float offset,
                                cudaStream_t st) {
   constexpr int VEC = Elem<T>::kVec;
   RowShape shape;
-  if (M % VEC == 0 && pick_row_shape(M / VEC, 8, &shape)) {
-    TYLO_ROW_DISPATCH(shape, norm_fwd_kernel<T, THREADS, ITERS, LAYER><<<(unsigned)N, THREADS, 0, st>>>(
-        (T*)Y, (const T*)X, (const T*)W, (const T*)Bias, Mean, Rstd, (int)M, eps, offset));
+  if (M % VEC == 0 && pick_row_shape(M / VEC, &shape)) {
+    TYLO_ROW_DISPATCH(shape, norm_fwd_kernel<T, THREADS, ITERS, LAYER><<<row_grid(THREADS, N), row_cta(THREADS), 0, st>>>(
+        (T*)Y, (const T*)X, (const T*)W, (const T*)Bias, Mean, Rstd, (int)M, (int)N, eps, offset));
   } else {
     norm_fwd_generic_kernel<T, LAYER><<<(unsigned)N, 256, 0, st>>>(
         (T*)Y, (const T*)X, (const T*)W, (const T*)Bias, Mean, Rstd, M, eps, offset);
@@ -522,37 +689,65 @@ static int32_t norm_bwd_launch(void* dX, void* dW, void* dB, const void* dY, con
                                float* dBp, int n_groups, int64_t M, int64_t N, float offset,
                                cudaStream_t st) {
   constexpr int VEC = Elem<T>::kVec;
-  RowShape shape;
-  unsigned grid = (unsigned)(n_groups < N ? n_groups : N);
+  const int sms = sm_count();
+  const char* what = LAYER ? "layer_norm_bwd" : "rms_norm_bwd";
   const int64_t nvec = M % VEC == 0 ? M / VEC : 0;
+  const int64_t acc_bytes = (LAYER ? 2 : 1) * M * 4;
+  auto walkers = [&](int64_t rows, int per_sm) {     // CTAs: no more than there are rows or partial rows, or fit at once
+    int64_t g = n_groups < rows ? n_groups : rows;
+    return (unsigned)(g < (int64_t)sms * per_sm ? g : (int64_t)sms * per_sm);
+  };
+  unsigned grid;
   if (nvec == 1024 || nvec == 512) {
-    // rows of exactly one packet per thread: the streaming form, one CTA per SM (two at 512 threads)
-    const unsigned walkers = (unsigned)sm_count() * (nvec == 1024 ? 1u : 2u);
-    if (grid > walkers) grid = walkers;
+    // one packet per thread and a CTA size known to the compiler: 64 registers without spills (rms 8192 bf16, 8,192 rows,
+    // forward + backward: 131 us; 164 us in the general form below)
+    grid = walkers(N, nvec == 1024 ? 1 : 2);
     if (nvec == 1024)
       norm_bwd_stream_kernel<T, 1024, LAYER><<<grid, 1024, 0, st>>>(
           (T*)dX, dWp, dBp, (const T*)dY, (const T*)X, (const T*)W, Mean, Rstd, (int)M, N, offset);
     else
       norm_bwd_stream_kernel<T, 512, LAYER><<<grid, 512, 0, st>>>(
           (T*)dX, dWp, dBp, (const T*)dY, (const T*)X, (const T*)W, Mean, Rstd, (int)M, N, offset);
-  } else
-  // register-resident shapes only while the per-thread dW/dB accumulators fit without spilling
-  if (M % VEC == 0 && M / VEC <= 1024 && pick_row_shape(M / VEC, 4, &shape)) {
-#define TYLO_BWD_LAUNCH(THREADS, ITERS)                                                             \
-  norm_bwd_kernel<T, THREADS, ITERS, LAYER><<<grid, THREADS, 0, st>>>(                              \
-      (T*)dX, dWp, dBp, (const T*)dY, (const T*)X, (const T*)W, Mean, Rstd, (int)M, N, offset)
-    if (shape.threads == 32) TYLO_BWD_LAUNCH(32, 2);
-    else if (shape.threads == 128) TYLO_BWD_LAUNCH(128, 2);
-    else TYLO_BWD_LAUNCH(256, 4);
-#undef TYLO_BWD_LAUNCH
+  } else if (nvec >= 1 && nvec <= 1024) {
+    const int tpr = (int)(nvec + 31) / 32 * 32;
+    // as many rows per CTA as make 512 threads, fewer when there are not enough rows to occupy every SM with that
+    int R = 512 / tpr;
+    if (R > kNormRowGroups) R = kNormRowGroups;
+    const int64_t per_sm = (N + sms - 1) / sms;
+    if (R > per_sm) R = (int)per_sm;
+    if (R < 1) R = 1;
+    grid = walkers((N + R - 1) / R, tpr * R > 512 ? 1 : 2);
+    const size_t smem = (size_t)R * 2 * 64 * 4 + (R > 1 ? acc_bytes : 0);
+    auto kern = nvec == tpr ? norm_bwd_kernel<T, LAYER, true> : norm_bwd_kernel<T, LAYER, false>;
+    // (several rows per CTA means rows of at most 256 packets: below the 48 KB that need no attribute)
+    kern<<<grid, tpr * R, smem, st>>>((T*)dX, dWp, dBp, (const T*)dY, (const T*)X, (const T*)W, Mean, Rstd, (int)M, (int)N,
+                                      offset, tpr, R);
+  } else if (nvec > 1024 && nvec <= 4096 && acc_bytes + 512 <= kMaxSmem) {
+    grid = walkers(N, 1);
+#define TYLO_BWD_WIDE(P)                                                                                              \
+  do {                                                                                                                \
+    auto kern = norm_bwd_wide_kernel<T, P, LAYER>;                                                                    \
+    if (int32_t rc = allow_smem(kern, acc_bytes + 512)) return rc;                                                    \
+    kern<<<grid, (unsigned)((nvec + P - 1) / P + 31) / 32 * 32, acc_bytes + 512, st>>>(                               \
+        (T*)dX, dWp, dBp, (const T*)dY, (const T*)X, (const T*)W, Mean, Rstd, (int)M, N, offset);                     \
+  } while (0)
+    if (nvec <= 2048) TYLO_BWD_WIDE(2); else TYLO_BWD_WIDE(4);
+#undef TYLO_BWD_WIDE
   } else {
-    norm_bwd_generic_kernel<T, LAYER><<<grid, 256, 0, st>>>(
-        (T*)dX, dWp, dBp, (const T*)dY, (const T*)X, (const T*)W, Mean, Rstd, M, N, offset);
+    const int64_t smem = acc_bytes + 2 * M * 4;
+    const int per_sm = smem <= kMaxSmem / 3 ? 3 : (smem <= kMaxSmem / 2 ? 2 : 1);
+    grid = walkers(N, smem <= kMaxSmem ? per_sm : 2);
+    if (smem <= kMaxSmem) {
+      auto kern = norm_bwd_generic_kernel<T, LAYER, true>;
+      if (int32_t rc = allow_smem(kern, smem)) return rc;
+      kern<<<grid, 512, smem, st>>>((T*)dX, dWp, dBp, (const T*)dY, (const T*)X, (const T*)W, Mean, Rstd, M, N, offset);
+    } else {
+      norm_bwd_generic_kernel<T, LAYER, false><<<grid, 512, 0, st>>>(
+          (T*)dX, dWp, dBp, (const T*)dY, (const T*)X, (const T*)W, Mean, Rstd, M, N, offset);
+    }
   }
-  int32_t rc = check_launch(LAYER ? "layer_norm_bwd" : "rms_norm_bwd");
-  if (rc) return rc;
-  norm_bwd_reduce_kernel<T><<<(unsigned)((M + 31) / 32), 256, 0, st>>>(
-      (T*)dW, (T*)dB, dWp, LAYER ? dBp : nullptr, M, (int)grid);
+  if (int32_t rc = check_launch(what)) return rc;
+  norm_bwd_reduce_kernel<T><<<(unsigned)((M + 31) / 32), 1024, 0, st>>>((T*)dW, (T*)dB, dWp, LAYER ? dBp : nullptr, M, (int)grid);
   return check_launch("norm_bwd_reduce");
 }
 

@@ -10,6 +10,55 @@
 
 namespace tylo {
 
+// A row that starts or ends inside a 16-byte packet (M not a multiple of the packet, so that rows of a 16-byte aligned array
+// start at every element offset).  Packets are counted from the aligned address at or before the row's start; all but the
+// first and the last are whole and move as 16 bytes, those two element by element, so nothing outside the row is touched.
+// Every array of a call is aligned alike, so one row has the same offset in all of them.
+template <typename T> struct RaggedRow {
+  static constexpr int kVec = Elem<T>::kVec;
+  T* row;
+  int off;                 // elements of packet 0 that lie before the row
+  int64_t M;
+  int nvec;
+  __device__ __forceinline__ RaggedRow(const T* r, int64_t m)
+      : row(const_cast<T*>(r)), off((int)((reinterpret_cast<uintptr_t>(r) & 15) / sizeof(T))), M(m), nvec((int)((off + m + kVec - 1) / kVec)) {}
+  __device__ __forceinline__ bool whole(int v) const { return (v > 0 || off == 0) && (int64_t)(v + 1) * kVec <= off + M; }
+  // packet v, elements outside the row (and packets past it) read as `fill`
+  __device__ __forceinline__ Pack<T> load(int v, float fill) const {
+    Pack<T> p;
+    if (v < nvec && whole(v)) { p.raw = ld_stream(row - off + (size_t)v * kVec); return p; }
+    float f[kVec];
+#pragma unroll
+    for (int j = 0; j < kVec; ++j) {
+      const int64_t i = (int64_t)v * kVec + j - off;
+      f[j] = (i >= 0 && i < M) ? Elem<T>::to_f(row[i]) : fill;
+    }
+    p.pack(f);
+    return p;
+  }
+  __device__ __forceinline__ void store(int v, const Pack<T>& p) const {
+    if (v >= nvec) return;
+    if (whole(v)) { st_stream(row - off + (size_t)v * kVec, p.raw); return; }
+    float f[kVec];
+    p.unpack(f);
+#pragma unroll
+    for (int j = 0; j < kVec; ++j) {
+      const int64_t i = (int64_t)v * kVec + j - off;
+      if (i >= 0 && i < M) row[i] = Elem<T>::from_f(f[j]);
+    }
+  }
+};
+
+// Rows of one warp share a CTA, eight at a time (a CTA of one warp per row leaves the SM at its limit of 32 CTAs, 32 warps, and
+// spends as long on starting CTAs as on the rows: 3.3 TB/s at 512 bf16 elements); longer rows have a CTA each.
+constexpr int kWarpRows = 8;
+constexpr int row_cta(int threads) { return threads == 32 ? 32 * kWarpRows : threads; }
+inline unsigned row_grid(int threads, int64_t rows) { return (unsigned)(threads == 32 ? (rows + kWarpRows - 1) / kWarpRows : rows); }
+template <int THREADS> __device__ __forceinline__ int row_thread() { return THREADS == 32 ? (int)(threadIdx.x & 31) : (int)threadIdx.x; }
+template <int THREADS> __device__ __forceinline__ size_t row_index() {
+  return THREADS == 32 ? (size_t)blockIdx.x * kWarpRows + (threadIdx.x >> 5) : (size_t)blockIdx.x;
+}
+
 template <typename T, int THREADS, int ITERS> struct RowRegs {
   static constexpr int kVec = Elem<T>::kVec;
   static constexpr int kMaxElems = THREADS * ITERS * kVec;
@@ -18,15 +67,23 @@ template <typename T, int THREADS, int ITERS> struct RowRegs {
   __device__ __forceinline__ void load(const T* __restrict__ row, int nvec) {
 #pragma unroll
     for (int i = 0; i < ITERS; ++i) {
-      const int v = i * THREADS + threadIdx.x;
+      const int v = i * THREADS + row_thread<THREADS>();
       if (v < nvec) p[i].raw = ld_stream(row + (size_t)v * kVec);
       else p[i].raw = make_uint4(0, 0, 0, 0);
     }
   }
+  __device__ __forceinline__ void load(const RaggedRow<T>& row, float fill) {
+#pragma unroll
+    for (int i = 0; i < ITERS; ++i) p[i] = row.load(i * THREADS + row_thread<THREADS>(), fill);
+  }
+  __device__ __forceinline__ void store(const RaggedRow<T>& row) const {
+#pragma unroll
+    for (int i = 0; i < ITERS; ++i) row.store(i * THREADS + row_thread<THREADS>(), p[i]);
+  }
   __device__ __forceinline__ void store(T* __restrict__ row, int nvec) const {
 #pragma unroll
     for (int i = 0; i < ITERS; ++i) {
-      const int v = i * THREADS + threadIdx.x;
+      const int v = i * THREADS + row_thread<THREADS>();
       if (v < nvec) st_stream(row + (size_t)v * kVec, p[i].raw);
     }
   }
@@ -39,15 +96,14 @@ template <typename T> __device__ __forceinline__ Pack<T> ld_param(const T* p) {
   return r;
 }
 
-// Launch-shape table shared by the row kernels: (threads, packets per thread).
-// Chosen so that each thread keeps 32-128 bytes of the row in flight.
+// Launch-shape table (threads, packets per thread) of the norm forwards: 32-128 bytes of the row in flight per thread, and
+// a shape for every power of two of packets up to 4,096, so that the common row lengths leave no thread idle (with 256 x 4
+// for 512 packets, half of them were: layer norm 4096 bf16 2.9 TB/s).
 struct RowShape { int threads, iters; };
-inline bool pick_row_shape(int64_t nvec, int max_iters, RowShape* out) {
-  static const RowShape table[] = {{32, 2}, {128, 2}, {256, 4}, {512, 8}, {1024, 8}};
-  for (const RowShape& s : table) {
-    if (s.iters <= max_iters && (int64_t)s.threads * s.iters >= nvec) { *out = s; return true; }
-  }
-  if (max_iters < 8 && nvec <= 1024 * (int64_t)max_iters) { *out = {1024, max_iters}; return true; }
+inline bool pick_row_shape(int64_t nvec, RowShape* out) {
+  static const RowShape table[] = {{32, 2}, {64, 2}, {128, 2}, {128, 4}, {256, 4}, {512, 4}, {512, 8}, {1024, 8}};
+  for (const RowShape& s : table)
+    if ((int64_t)s.threads * s.iters >= nvec) { *out = s; return true; }
   return false;
 }
 
