@@ -1,0 +1,65 @@
+"""GPU parity: the row kernels at the edges of their launch shapes — rows that start inside a 16-byte packet, rows too long
+for one CTA's registers, norm backward with several rows per CTA, with more than one packet per thread, and with fewer
+partial rows or tokens than CTAs."""
+import numpy as np
+import pytest
+import torch
+
+from gpu_util import back, check, draw
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dt", ["f32", "bf16", "f16"])
+@pytest.mark.parametrize("M,N", [(1, 5), (7, 9), (9, 3), (63, 4), (513, 3), (2049, 3), (4095, 3), (8193, 2), (65533, 2), (65544, 2),
+                                 (70001, 2), (131072, 1)])
+def test_softmax_rows(tylo, oracle, M, N, dt):
+    rng = np.random.default_rng(M + N)
+    buf = torch.full((N * M + 32,), 7.0, device="cuda", dtype={"f32": torch.float32, "bf16": torch.bfloat16, "f16": torch.float16}[dt])
+    X, X64 = draw(rng, (N, M), dt, scale=2.0)
+    Y = buf[:N * M].view(N, M)
+    tylo.softmax_(Y, X)
+    assert bool((buf[N * M:] == 7.0).all())          # nothing beyond the last row is written
+    check(Y, oracle.softmax_ref(X64), dt, "softmax")
+    dY, dY64 = draw(rng, (N, M), dt)
+    check(tylo.grad_softmax(dY, Y), oracle.softmax_bwd_ref(dY64, back(Y)), dt, "softmax bwd")
+
+
+@pytest.mark.parametrize("M", [9, 4097, 70001, 131072])
+def test_softmax_minus_infinity(tylo, oracle, M):
+    X = torch.randn(3, M, device="cuda")
+    X[0, 1:] = float("-inf")                          # one entry left
+    X[1, ::2] = float("-inf")
+    X[2, :-1] = float("-inf")
+    check(tylo.softmax(X), oracle.softmax_ref(back(X)), "f32", "softmax")
+
+
+# packets per row (f32: 4 elements, 16-bit: 8): one warp, a warp and one, eight rows per CTA, ragged thread counts, 1,024 and
+# beyond (two and four packets per thread), and lengths that are not a multiple of the packet
+@pytest.mark.parametrize("dt", ["f32", "bf16"])
+@pytest.mark.parametrize("M,N,groups", [(8, 40, 296), (256, 700, 296), (264, 31, 3), (520, 5000, 296), (4104, 301, 296), (8192, 3, 1),
+                                        (8200, 17, 5), (12288, 200, 296), (16384, 9, 296), (16392, 3, 296), (1, 7, 296), (1001, 333, 296),
+                                        (33001, 2, 296)])
+def test_norm_rows(tylo, oracle, M, N, groups, dt):
+    rng = np.random.default_rng(M + N)
+    eps = 1e-5
+    X, X64 = draw(rng, (N, M), dt, shift=0.3)
+    W, W64 = draw(rng, (M,), dt, scale=0.1, shift=1.0)
+    B, B64 = draw(rng, (M,), dt, scale=0.1)
+    dY, dY64 = draw(rng, (N, M), dt)
+    cp = tylo.allocate_checkpoints_rms_norm(X, W)
+    check(tylo.rms_norm(X, W, eps=eps, offset=0.25, checkpoints=cp), oracle.rms_norm_ref(X64, W64, eps=eps, offset=0.25), dt, "rms")
+    sc = tylo.allocate_scratchspace_grad_rms_norm(X, W, N_GROUPS=groups)
+    dX, dW = tylo.grad_rms_norm(dY, X, W, checkpoints=cp, offset=0.25, scratch=sc)
+    dXr, dWr, _ = oracle.rms_norm_bwd_ref(dY64, X64, W64, eps=eps, offset=0.25)
+    check(dX, dXr, dt, "rms dX"); check(dW, dWr, dt, "rms dW", scale_hint=4 * float(np.abs(dWr).max()))
+    if M == 1:
+        return                                        # LayerNorm of one element: 0 / sqrt(eps) against rounding noise
+    cpl = tylo.allocate_checkpoints_layer_norm(X, W, B)
+    check(tylo.layer_norm(X, W, B, eps=eps, checkpoints=cpl), oracle.layer_norm_ref(X64, W64, B64, eps=eps), dt, "ln")
+    sc = tylo.allocate_scratchspace_grad_layer_norm(X, W, B, N_GROUPS=groups)
+    dX, dW, dB = tylo.grad_layer_norm(dY, X, W, B, checkpoints=cpl, scratch=sc)
+    dXr, dWr, dBr, _, _ = oracle.layer_norm_bwd_ref(dY64, X64, W64, eps=eps)
+    check(dX, dXr, dt, "ln dX")
+    check(dW, dWr, dt, "ln dW", scale_hint=4 * float(np.abs(dWr).max()))
+    check(dB, dBr, dt, "ln dB", scale_hint=4 * float(np.abs(dBr).max()))

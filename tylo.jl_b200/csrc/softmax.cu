@@ -1,28 +1,22 @@
 // Row softmax forward / backward for sm_100a: one read and one write of HBM per element
 // (the reference's streaming kernel reads X twice, softmax.jl:6-33).
 //
-// A row of up to 8192 (16-bit) / 4096 (fp32) elements is held in the registers of one CTA.
-// Longer rows are split across a thread-block cluster of 2, 4 or 8 CTAs whose partial
-// (max, sum) pairs are exchanged through distributed shared memory, so that several
-// part-rows are resident per SM and their load, exp and store phases overlap.
+// A row of up to 32,768 (16-bit) / 8,192 (fp32) elements (forward; 8,192 / 4,096 backward) is held in the registers of one
+// CTA, or of one warp when it is short; longer rows take two passes, the second of which reads out of L2.  Rows of any
+// length and start move as 16-byte packets (see RaggedRow).
 //
 // exp is evaluated once per element: each thread first takes the max of its own elements,
 // exponentiates against that, and the result is rescaled by exp2(m_thread - m_row) / sum
 // — one extra exp per thread instead of one per element.
-#include <cooperative_groups.h>
-
 #include "rowwise.cuh"
-
-namespace cg = cooperative_groups;
 
 namespace tylo {
 
 constexpr float kLog2e = 1.4426950408889634f;
 
-// Combine a per-thread (max, sum-relative-to-that-max) pair over the CTA and, when CLUSTER > 1,
-// over the cluster.  Returns the row max and the row sum relative to it.
-template <int THREADS, bool CLUSTERED>
-__device__ __forceinline__ void reduce_max_sum(float& m, float& s, float* smem /* >= 80 floats */) {
+// Combine a per-thread (max, sum-relative-to-that-max) pair over the row's threads.  Returns the row max and the row sum relative to it.
+template <int THREADS>
+__device__ __forceinline__ void reduce_max_sum(float& m, float& s, float* smem /* >= 64 floats */) {
   // warp level
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -45,75 +39,33 @@ __device__ __forceinline__ void reduce_max_sum(float& m, float& s, float* smem /
       m = mn;
     }
   }
-  if constexpr (CLUSTERED) {
-    cg::cluster_group cluster = cg::this_cluster();
-    __syncthreads();
-    if (threadIdx.x == 0) { smem[64] = m; smem[65] = s; }
-    cluster.sync();
-    const unsigned n = cluster.num_blocks();
-    float mr = -INFINITY, sr = 0.f;
-    if (lane < (int)n) {
-      const float* peer = cluster.map_shared_rank(smem, lane);
-      mr = peer[64]; sr = peer[65];
-    }
-#pragma unroll
-    for (int o = 4; o > 0; o >>= 1) {  // cluster size <= 8
-      const float m2 = __shfl_xor_sync(0xffffffffu, mr, o), s2 = __shfl_xor_sync(0xffffffffu, sr, o);
-      const float mn = fmaxf(mr, m2);
-      sr = (mn == -INFINITY) ? 0.f : sr * exp2f(mr - mn) + s2 * exp2f(m2 - mn);
-      mr = mn;
-    }
-    m = __shfl_sync(0xffffffffu, mr, 0);
-    s = __shfl_sync(0xffffffffu, sr, 0);
-    cluster.sync();  // peers may exit (and release their shared memory) only after all reads
-  } else if constexpr (THREADS > 32) {
-    __syncthreads();
-  }
+  if constexpr (THREADS > 32) __syncthreads();
 }
 
-template <int THREADS, bool CLUSTERED>
-__device__ __forceinline__ float reduce_sum(float v, float* smem) {
-  v = block_reduce<THREADS>(v, SumOp(), 0.f, smem);
-  if constexpr (CLUSTERED) {
-    cg::cluster_group cluster = cg::this_cluster();
-    if (threadIdx.x == 0) smem[64] = v;
-    cluster.sync();
-    const unsigned n = cluster.num_blocks();
-    const int lane = threadIdx.x & 31;
-    float r = 0.f;
-    if (lane < (int)n) r = cluster.map_shared_rank(smem, lane)[64];
-#pragma unroll
-    for (int o = 4; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
-    v = __shfl_sync(0xffffffffu, r, 0);
-    cluster.sync();
-  }
-  return v;
-}
-
-template <typename T, int THREADS, int ITERS, bool CLUSTERED>
-__global__ void __launch_bounds__(THREADS)
-softmax_fwd_kernel(T* __restrict__ Y, const T* __restrict__ X, int64_t M, int part_elems) {
+template <typename T, int THREADS, int ITERS, bool RAGGED>
+__global__ void __launch_bounds__(row_cta(THREADS))
+softmax_fwd_kernel(T* __restrict__ Y, const T* __restrict__ X, int64_t M, int N) {
   constexpr int VEC = Elem<T>::kVec;
-  __shared__ float smem[80];
-  unsigned csize = 1, crank = 0;
-  if constexpr (CLUSTERED) {
-    cg::cluster_group cluster = cg::this_cluster();
-    csize = cluster.num_blocks(); crank = cluster.block_rank();
-  }
-  const size_t row = blockIdx.x / csize;
-  const int64_t begin = (int64_t)crank * part_elems;
-  int64_t len = M - begin; if (len > part_elems) len = part_elems; if (len < 0) len = 0;
-  const int nvec = (int)(len / VEC);
-  const T* x = X + row * M + begin;
+  __shared__ float smem[64];
+  const size_t row = row_index<THREADS>();
+  if (THREADS == 32 && row >= (size_t)N) return;
+  const int tid = row_thread<THREADS>();
+  int nvec = (int)(M / VEC);
 
   RowRegs<T, THREADS, ITERS> r;
-  r.load(x, nvec);
+  if constexpr (RAGGED) {
+    const RaggedRow<T> x(X + row * M, M);
+    nvec = (int)x.nvec;
+    r.load(x, -INFINITY);
+  } else {
+    r.load(X + row * M, nvec);
+  }
   float e[ITERS][VEC];
   float m = -INFINITY;
 #pragma unroll
   for (int i = 0; i < ITERS; ++i) {
     r.p[i].unpack(e[i]);
-    if (i * THREADS + (int)threadIdx.x < nvec) {
+    if (i * THREADS + tid < nvec) {
 #pragma unroll
       for (int j = 0; j < VEC; ++j) m = fmaxf(m, e[i][j]);
     }
@@ -123,7 +75,7 @@ softmax_fwd_kernel(T* __restrict__ Y, const T* __restrict__ X, int64_t M, int pa
   float s = 0.f;
 #pragma unroll
   for (int i = 0; i < ITERS; ++i) {
-    const bool live = i * THREADS + (int)threadIdx.x < nvec;
+    const bool live = i * THREADS + tid < nvec;
 #pragma unroll
     for (int j = 0; j < VEC; ++j) {
       e[i][j] = live ? exp2f((e[i][j] - mt) * kLog2e) : 0.f;
@@ -131,7 +83,7 @@ softmax_fwd_kernel(T* __restrict__ Y, const T* __restrict__ X, int64_t M, int pa
     }
   }
   m *= kLog2e;  // reductions run in log2 units
-  reduce_max_sum<THREADS, CLUSTERED>(m, s, smem);
+  reduce_max_sum<THREADS>(m, s, smem);
   // a row made only of -Inf yields zeros (nothing in the reference's tests pins that case)
   const float factor = (m_thread == -INFINITY) ? 0.f : exp2f(m_thread * kLog2e - m) / s;
 #pragma unroll
@@ -140,7 +92,8 @@ softmax_fwd_kernel(T* __restrict__ Y, const T* __restrict__ X, int64_t M, int pa
     for (int j = 0; j < VEC; ++j) e[i][j] *= factor;
     r.p[i].pack(e[i]);
   }
-  r.store(Y + row * M + begin, nvec);
+  if constexpr (RAGGED) r.store(RaggedRow<T>(Y + row * M, M));
+  else r.store(Y + row * M, nvec);
 }
 
 __device__ __forceinline__ float ex2_fast(float x) {
@@ -153,19 +106,29 @@ __device__ __forceinline__ float ex2_fast(float x) {
 // registers of an fp32 copy, so twice the bytes in flight per SM for the same occupancy) and exp is
 // evaluated twice per element (once for the sum, once for the output) on the otherwise idle
 // special-function unit; its approximate form is ample for a 16-bit result.
-template <typename T, int THREADS, int ITERS>
-__global__ void __launch_bounds__(THREADS)
-softmax_fwd_packed_kernel(T* __restrict__ Y, const T* __restrict__ X, int64_t M) {
+// (at 16 packets per thread three CTAs per SM are asked for: 80 registers; left alone the compiler takes 128, and 2048 rows
+// of 32,768 bf16 go from 51 to 57 us)
+template <typename T, int THREADS, int ITERS, bool RAGGED>
+__global__ void __launch_bounds__(row_cta(THREADS), ITERS == 16 ? 3 : 1)
+softmax_fwd_packed_kernel(T* __restrict__ Y, const T* __restrict__ X, int64_t M, int N) {
   constexpr int VEC = Elem<T>::kVec;
   __shared__ float smem[32];
-  const int nvec = (int)(M / VEC);
-  const size_t row = blockIdx.x;
+  int nvec = (int)(M / VEC);
+  const size_t row = row_index<THREADS>();
+  if (THREADS == 32 && row >= (size_t)N) return;
+  const int tid = row_thread<THREADS>();
   RowRegs<T, THREADS, ITERS> r;
-  r.load(X + row * M, nvec);
+  if constexpr (RAGGED) {
+    const RaggedRow<T> x(X + row * M, M);
+    nvec = (int)x.nvec;
+    r.load(x, -INFINITY);
+  } else {
+    r.load(X + row * M, nvec);
+  }
   float m = -INFINITY;
 #pragma unroll
   for (int i = 0; i < ITERS; ++i) {
-    if (i * THREADS + (int)threadIdx.x < nvec) {
+    if (i * THREADS + tid < nvec) {
       float f[VEC]; r.p[i].unpack(f);
 #pragma unroll
       for (int j = 0; j < VEC; ++j) m = fmaxf(m, f[j]);
@@ -176,7 +139,7 @@ softmax_fwd_packed_kernel(T* __restrict__ Y, const T* __restrict__ X, int64_t M)
   float s = 0.f;
 #pragma unroll
   for (int i = 0; i < ITERS; ++i) {
-    if (i * THREADS + (int)threadIdx.x < nvec) {
+    if (i * THREADS + tid < nvec) {
       float f[VEC]; r.p[i].unpack(f);
 #pragma unroll
       for (int j = 0; j < VEC; ++j) s += ex2_fast(fmaf(f[j], kLog2e, -mo));
@@ -191,28 +154,92 @@ softmax_fwd_packed_kernel(T* __restrict__ Y, const T* __restrict__ X, int64_t M)
     for (int j = 0; j < VEC; ++j) f[j] = ex2_fast(fmaf(f[j], kLog2e, -mo)) * inv;
     r.p[i].pack(f);
   }
-  r.store(Y + row * M, nvec);
+  if constexpr (RAGGED) r.store(RaggedRow<T>(Y + row * M, M));
+  else r.store(Y + row * M, nvec);
 }
 
-template <typename T, int THREADS, int ITERS, bool CLUSTERED>
+// Rows too long for one CTA's registers, forward: a pass that keeps a running (max, sum) per thread and a pass that reads
+// the row again out of L2 (see the backward's two-pass form below) and writes.
+template <typename T, int THREADS, bool RAGGED>
 __global__ void __launch_bounds__(THREADS)
-softmax_bwd_kernel(T* __restrict__ dX, const T* __restrict__ dY, const T* __restrict__ Y, int64_t M,
-                   int part_elems) {
-  constexpr int VEC = Elem<T>::kVec;
-  __shared__ float smem[80];
-  unsigned csize = 1, crank = 0;
-  if constexpr (CLUSTERED) {
-    cg::cluster_group cluster = cg::this_cluster();
-    csize = cluster.num_blocks(); crank = cluster.block_rank();
+softmax_fwd_twopass_kernel(T* __restrict__ Y, const T* __restrict__ X, int64_t M) {
+  constexpr int VEC = Elem<T>::kVec, U = 4;
+  __shared__ float smem[64];
+  const size_t base = (size_t)blockIdx.x * M;
+  const RaggedRow<T> x(X + base, M), y(Y + base, M);
+  const int nvec = RAGGED ? x.nvec : (int)(M / VEC);
+  auto ex2 = [](float v) { return sizeof(T) == 2 ? ex2_fast(v) : exp2f(v); };
+  auto load = [&](int v) {
+    Pack<T> p;
+    if constexpr (RAGGED) return x.load(v, -INFINITY);
+    if (v < nvec) { p.raw = __ldg(reinterpret_cast<const uint4*>(X + base) + v); return p; }
+    float f[VEC];
+#pragma unroll
+    for (int j = 0; j < VEC; ++j) f[j] = -INFINITY;
+    p.pack(f);
+    return p;
+  };
+  float m = -INFINITY, s = 0.f;        // m in log2 units
+  for (int v0 = threadIdx.x; v0 < nvec; v0 += U * THREADS) {
+    Pack<T> p[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) p[u] = load(v0 + u * THREADS);
+    float mx = -INFINITY;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      float f[VEC]; p[u].unpack(f);
+#pragma unroll
+      for (int j = 0; j < VEC; ++j) mx = fmaxf(mx, f[j]);
+    }
+    const float mn = fmaxf(m, mx * kLog2e);
+    if (mn != -INFINITY) {
+      s *= ex2(m - mn);
+      m = mn;
+    }
+    const float mo = m == -INFINITY ? 0.f : m;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      float f[VEC]; p[u].unpack(f);
+#pragma unroll
+      for (int j = 0; j < VEC; ++j) s += ex2(fmaf(f[j], kLog2e, -mo));
+    }
   }
-  const size_t row = blockIdx.x / csize;
-  const int64_t begin = (int64_t)crank * part_elems;
-  int64_t len = M - begin; if (len > part_elems) len = part_elems; if (len < 0) len = 0;
-  const int nvec = (int)(len / VEC);
+  reduce_max_sum<THREADS>(m, s, smem);
+  const float inv = m == -INFINITY ? 0.f : 1.f / s, mo = m == -INFINITY ? 0.f : m;
+  for (int v0 = threadIdx.x; v0 < nvec; v0 += U * THREADS) {
+    Pack<T> p[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) p[u] = load(v0 + u * THREADS);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int v = v0 + u * THREADS;
+      float f[VEC]; p[u].unpack(f);
+#pragma unroll
+      for (int j = 0; j < VEC; ++j) f[j] = ex2(fmaf(f[j], kLog2e, -mo)) * inv;
+      p[u].pack(f);
+      if constexpr (RAGGED) y.store(v, p[u]);
+      else if (v < nvec) st_stream(Y + base + (size_t)v * VEC, p[u].raw);
+    }
+  }
+}
+
+template <typename T, int THREADS, int ITERS, bool RAGGED>
+__global__ void __launch_bounds__(row_cta(THREADS))
+softmax_bwd_kernel(T* __restrict__ dX, const T* __restrict__ dY, const T* __restrict__ Y, int64_t M, int N) {
+  constexpr int VEC = Elem<T>::kVec;
+  __shared__ float smem[32];
+  const size_t row = row_index<THREADS>();
+  if (THREADS == 32 && row >= (size_t)N) return;
+  const int nvec = (int)(M / VEC);
 
   RowRegs<T, THREADS, ITERS> y, dy;
-  y.load(Y + row * M + begin, nvec);
-  dy.load(dY + row * M + begin, nvec);
+  if constexpr (RAGGED) {
+    y.load(RaggedRow<T>(Y + row * M, M), 0.f);
+    dy.load(RaggedRow<T>(dY + row * M, M), 0.f);
+  } else {
+    y.load(Y + row * M, nvec);
+    dy.load(dY + row * M, nvec);
+  }
   float dot = 0.f;
 #pragma unroll
   for (int i = 0; i < ITERS; ++i) {
@@ -221,7 +248,7 @@ softmax_bwd_kernel(T* __restrict__ dX, const T* __restrict__ dY, const T* __rest
 #pragma unroll
     for (int j = 0; j < VEC; ++j) dot += a[j] * b[j];
   }
-  dot = reduce_sum<THREADS, CLUSTERED>(dot, smem);
+  dot = block_reduce<THREADS>(dot, SumOp(), 0.f, smem);
 #pragma unroll
   for (int i = 0; i < ITERS; ++i) {
     float a[VEC], b[VEC];
@@ -230,33 +257,35 @@ softmax_bwd_kernel(T* __restrict__ dX, const T* __restrict__ dY, const T* __rest
     for (int j = 0; j < VEC; ++j) a[j] = a[j] * (b[j] - dot);
     y.p[i].pack(a);
   }
-  y.store(dX + row * M + begin, nvec);
+  if constexpr (RAGGED) y.store(RaggedRow<T>(dX + row * M, M));
+  else y.store(dX + row * M, nvec);
 }
 
 // Long rows, backward: two passes over Y and dY instead of a register-resident row.  Pass 1 sums y * dy, pass 2
 // reads both again — a row pair is 128 KB at 32,768 16-bit elements, a few hundred of them in flight fit L2 many
 // times over, so the second read never reaches HBM — and writes dX.  No cluster, no row held in registers: a thread
 // keeps eight 16-byte loads in flight and the CTA is free of the all-or-nothing scheduling of a cluster.
-template <typename T, int THREADS>
+template <typename T, int THREADS, bool RAGGED>
 __global__ void __launch_bounds__(THREADS)
 softmax_bwd_twopass_kernel(T* __restrict__ dX, const T* __restrict__ dY, const T* __restrict__ Y, int64_t M) {
-  constexpr int VEC = Elem<T>::kVec;
+  constexpr int VEC = Elem<T>::kVec, U = 4;
   __shared__ float smem[32];
   const size_t base = (size_t)blockIdx.x * M;
-  const int nvec = (int)(M / VEC);
-  const uint4* y4 = reinterpret_cast<const uint4*>(Y + base);
-  const uint4* d4 = reinterpret_cast<const uint4*>(dY + base);
+  const RaggedRow<T> ry(Y + base, M), rd(dY + base, M), ro(dX + base, M);
+  const int nvec = RAGGED ? ry.nvec : (int)(M / VEC);
+  auto load = [&](const T* p, const RaggedRow<T>& r, int v) {
+    Pack<T> k;
+    if constexpr (RAGGED) return r.load(v, 0.f);
+    k.raw = v < nvec ? __ldg(reinterpret_cast<const uint4*>(p + base) + v) : make_uint4(0, 0, 0, 0);
+    return k;
+  };
   float dot = 0.f;
-  for (int v0 = threadIdx.x; v0 < nvec; v0 += 4 * THREADS) {
-    Pack<T> y[4], d[4];
+  for (int v0 = threadIdx.x; v0 < nvec; v0 += U * THREADS) {
+    Pack<T> y[U], d[U];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int v = v0 + u * THREADS;
-      y[u].raw = v < nvec ? __ldg(y4 + v) : make_uint4(0, 0, 0, 0);
-      d[u].raw = v < nvec ? __ldg(d4 + v) : make_uint4(0, 0, 0, 0);
-    }
+    for (int u = 0; u < U; ++u) { y[u] = load(Y, ry, v0 + u * THREADS); d[u] = load(dY, rd, v0 + u * THREADS); }
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
+    for (int u = 0; u < U; ++u) {
       float a[VEC], b[VEC];
       y[u].unpack(a); d[u].unpack(b);
 #pragma unroll
@@ -264,134 +293,56 @@ softmax_bwd_twopass_kernel(T* __restrict__ dX, const T* __restrict__ dY, const T
     }
   }
   dot = block_reduce<THREADS>(dot, SumOp(), 0.f, smem);
-  for (int v0 = threadIdx.x; v0 < nvec; v0 += 4 * THREADS) {
-    Pack<T> y[4], d[4];
+  for (int v0 = threadIdx.x; v0 < nvec; v0 += U * THREADS) {
+    Pack<T> y[U], d[U];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int v = v0 + u * THREADS;
-      y[u].raw = v < nvec ? __ldg(y4 + v) : make_uint4(0, 0, 0, 0);
-      d[u].raw = v < nvec ? __ldg(d4 + v) : make_uint4(0, 0, 0, 0);
-    }
+    for (int u = 0; u < U; ++u) { y[u] = load(Y, ry, v0 + u * THREADS); d[u] = load(dY, rd, v0 + u * THREADS); }
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
+    for (int u = 0; u < U; ++u) {
       const int v = v0 + u * THREADS;
       float a[VEC], b[VEC];
       y[u].unpack(a); d[u].unpack(b);
 #pragma unroll
       for (int j = 0; j < VEC; ++j) a[j] = a[j] * (b[j] - dot);
       y[u].pack(a);
-      if (v < nvec) st_stream(dX + base + (size_t)v * VEC, y[u].raw);
+      if constexpr (RAGGED) ro.store(v, y[u]);
+      else if (v < nvec) st_stream(dX + base + (size_t)v * VEC, y[u].raw);
     }
   }
 }
 
-// Any M, any alignment: online max/sum pass, then a second pass that re-reads X (mostly from L2).
-template <typename T>
-__global__ void __launch_bounds__(256)
-softmax_fwd_generic_kernel(T* __restrict__ Y, const T* __restrict__ X, int64_t M) {
-  __shared__ float smem[80];
-  const T* x = X + (size_t)blockIdx.x * M;
-  float m = -INFINITY, s = 0.f;
-  for (int64_t i = threadIdx.x; i < M; i += 256) {
-    const float v = Elem<T>::to_f(x[i]) * kLog2e;
-    const float mn = fmaxf(m, v);
-    s = (mn == -INFINITY) ? 0.f : s * exp2f(m - mn) + exp2f(v - mn);
-    m = mn;
-  }
-  reduce_max_sum<256, false>(m, s, smem);
-  const float inv = 1.0f / s;
-  for (int64_t i = threadIdx.x; i < M; i += 256)
-    Y[(size_t)blockIdx.x * M + i] = Elem<T>::from_f(exp2f(Elem<T>::to_f(x[i]) * kLog2e - m) * inv);
-}
-
-template <typename T>
-__global__ void __launch_bounds__(256)
-softmax_bwd_generic_kernel(T* __restrict__ dX, const T* __restrict__ dY, const T* __restrict__ Y, int64_t M) {
-  __shared__ float smem[32];
-  const size_t base = (size_t)blockIdx.x * M;
-  float dot = 0.f;
-  for (int64_t i = threadIdx.x; i < M; i += 256) dot += Elem<T>::to_f(Y[base + i]) * Elem<T>::to_f(dY[base + i]);
-  dot = block_reduce<256>(dot, SumOp(), 0.f, smem);
-  for (int64_t i = threadIdx.x; i < M; i += 256)
-    dX[base + i] = Elem<T>::from_f(Elem<T>::to_f(Y[base + i]) * (Elem<T>::to_f(dY[base + i]) - dot));
-}
-
-template <typename K, typename... Args>
-static int32_t launch_clustered(K kernel, unsigned grid, unsigned threads, unsigned cluster, cudaStream_t st,
-                                const char* what, Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid); cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = 0; cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = cluster; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr; cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
-  if (e != cudaSuccess) {
-    set_error("launch of %s failed: %s", what, cudaGetErrorString(e));
-    return TYLO_ERR_CUDA;
-  }
-  return TYLO_OK;
-}
-
-template <typename T, bool FWD>
+template <typename T, bool FWD, bool RAGGED>
 static int32_t softmax_launch(void* out, const void* a, const void* b, int64_t M, int64_t N, cudaStream_t st) {
   constexpr int VEC = Elem<T>::kVec;
-  constexpr int kPartVec = 256 * 4;  // packets per CTA in the clustered shape
   const char* what = FWD ? "softmax_fwd" : "softmax_bwd";
+  const int64_t nvec = RAGGED ? (M + 2 * VEC - 2) / VEC : M / VEC;     // packets a row may touch
+  // register-resident rows; a shape for every power of two of packets (see pick_row_shape)
+#define TYLO_SM_LAUNCH(THREADS, ITERS)                                                                               \
+  do {                                                                                                               \
+    const unsigned grid = row_grid(THREADS, N), cta = row_cta(THREADS);                                              \
+    if constexpr (!FWD) softmax_bwd_kernel<T, THREADS, ITERS, RAGGED><<<grid, cta, 0, st>>>(                         \
+        (T*)out, (const T*)a, (const T*)b, M, (int)N);                                                               \
+    else if constexpr (VEC == 8) softmax_fwd_packed_kernel<T, THREADS, ITERS, RAGGED><<<grid, cta, 0, st>>>(         \
+        (T*)out, (const T*)a, M, (int)N);                                                                            \
+    else softmax_fwd_kernel<T, THREADS, ITERS, RAGGED><<<grid, cta, 0, st>>>((T*)out, (const T*)a, M, (int)N);       \
+    return check_launch(what);                                                                                       \
+  } while (0)
+  if (nvec <= 64) TYLO_SM_LAUNCH(32, 2);
+  if (nvec <= 128) TYLO_SM_LAUNCH(64, 2);
+  if (nvec <= 256) TYLO_SM_LAUNCH(128, 2);
+  if (nvec <= 512) TYLO_SM_LAUNCH(128, 4);
+  if (nvec <= 1024) TYLO_SM_LAUNCH(256, 4);
   if constexpr (FWD && VEC == 8) {
-    if (M % VEC == 0 && M / VEC <= 512 * 16) {
-      const int64_t nv = M / VEC;
-#define TYLO_SMP(THREADS, ITERS)                                                                             \
-  do {                                                                                                       \
-    softmax_fwd_packed_kernel<T, THREADS, ITERS><<<(unsigned)N, THREADS, 0, st>>>((T*)out, (const T*)a, M);  \
-    return check_launch(what);                                                                               \
-  } while (0)
-      if (nv <= 64) TYLO_SMP(32, 2);
-      if (nv <= 256) TYLO_SMP(128, 2);
-      if (nv <= 1024) TYLO_SMP(256, 4);
-      if (nv <= 2048) TYLO_SMP(256, 8);
-      if (nv <= 4096) TYLO_SMP(256, 16);
-      TYLO_SMP(512, 16);
-#undef TYLO_SMP
-    }
+    if (nvec <= 2048) TYLO_SM_LAUNCH(256, 8);
+    if (nvec <= 4096) TYLO_SM_LAUNCH(256, 16);
+  } else if constexpr (FWD) {
+    if (nvec <= 2048) TYLO_SM_LAUNCH(512, 4);
   }
-  if (M % VEC == 0) {
-    const int64_t nvec = M / VEC;
-#define TYLO_SM_LAUNCH(THREADS, ITERS)                                                                      \
-  do {                                                                                                       \
-    if constexpr (FWD) softmax_fwd_kernel<T, THREADS, ITERS, false><<<(unsigned)N, THREADS, 0, st>>>(          \
-        (T*)out, (const T*)a, M, (int)M);                                                                    \
-    else softmax_bwd_kernel<T, THREADS, ITERS, false><<<(unsigned)N, THREADS, 0, st>>>(                        \
-        (T*)out, (const T*)a, (const T*)b, M, (int)M);                                                       \
-    return check_launch(what);                                                                               \
-  } while (0)
-    if (nvec <= 64) TYLO_SM_LAUNCH(32, 2);
-    if (nvec <= 256) TYLO_SM_LAUNCH(128, 2);
-    if (nvec <= kPartVec) TYLO_SM_LAUNCH(256, 4);
 #undef TYLO_SM_LAUNCH
-    if constexpr (!FWD) {
-      // rows too long for one CTA's registers: the two-pass form (4,952 GB/s with the clustered register-resident
-      // form on 4096 x 32768 bf16, 6,225 with this one at 1,024 threads; 5,317 at 512 and 4,042 at 256 threads)
-      if (nvec > kPartVec) {
-        softmax_bwd_twopass_kernel<T, 1024><<<(unsigned)N, 1024, 0, st>>>((T*)out, (const T*)a, (const T*)b, M);
-        return check_launch(what);
-      }
-    }
-    if (nvec <= 8 * kPartVec && N * 8 <= 0x7fffffffLL) {
-      unsigned c = 2;
-      while ((int64_t)c * kPartVec < nvec) c *= 2;
-      // even split, rounded up to whole packets
-      const int part = (int)(((nvec + c - 1) / c) * VEC);
-      if constexpr (FWD)
-        return launch_clustered(softmax_fwd_kernel<T, 256, 4, true>, (unsigned)(N * c), 256, c, st, what,
-                                (T*)out, (const T*)a, M, part);
-      else
-        return launch_clustered(softmax_bwd_kernel<T, 256, 4, true>, (unsigned)(N * c), 256, c, st, what,
-                                (T*)out, (const T*)a, (const T*)b, M, part);
-    }
-  }
-  if constexpr (FWD) softmax_fwd_generic_kernel<T><<<(unsigned)N, 256, 0, st>>>((T*)out, (const T*)a, M);
-  else softmax_bwd_generic_kernel<T><<<(unsigned)N, 256, 0, st>>>((T*)out, (const T*)a, (const T*)b, M);
+  // rows too long for one CTA's registers: the two-pass form (backward of 4096 x 32768 bf16: 4,952 GB/s with a clustered
+  // register-resident form, 6,225 with this one at 1,024 threads; 5,317 at 512 and 4,042 at 256 threads)
+  if constexpr (FWD) softmax_fwd_twopass_kernel<T, 1024, RAGGED><<<(unsigned)N, 1024, 0, st>>>((T*)out, (const T*)a, M);
+  else softmax_bwd_twopass_kernel<T, 1024, RAGGED><<<(unsigned)N, 1024, 0, st>>>((T*)out, (const T*)a, (const T*)b, M);
   return check_launch(what);
 }
 
@@ -406,7 +357,8 @@ extern "C" int32_t tylo_b200_softmax_fwd(void* Y, const void* X, int64_t M, int6
                (long long)M, (long long)N);
   TYLO_REQUIRE(N <= 0x7fffffffLL, TYLO_ERR_UNSUPPORTED, "softmax_fwd: N above 2^31-1 is not supported");
   TYLO_REQUIRE(aligned16(Y) && aligned16(X), TYLO_ERR_MISALIGNED, "softmax_fwd: pointers must be 16-byte aligned");
-  TYLO_DISPATCH_DTYPE(dtype, T, return (softmax_launch<T, true>(Y, X, nullptr, M, N, (cudaStream_t)stream)));
+  TYLO_DISPATCH_DTYPE(dtype, T, return (M % Elem<T>::kVec ? softmax_launch<T, true, true>(Y, X, nullptr, M, N, (cudaStream_t)stream)
+                                                       : softmax_launch<T, true, false>(Y, X, nullptr, M, N, (cudaStream_t)stream)));
   return TYLO_OK;
 }
 
@@ -419,6 +371,7 @@ extern "C" int32_t tylo_b200_softmax_bwd(void* dX, const void* dY, const void* Y
   TYLO_REQUIRE(aligned16(dX) && aligned16(dY) && aligned16(Y), TYLO_ERR_MISALIGNED,
                "softmax_bwd: pointers must be 16-byte aligned");
   // argument order of the kernel: (dX, dY, Y)
-  TYLO_DISPATCH_DTYPE(dtype, T, return (softmax_launch<T, false>(dX, dY, Y, M, N, (cudaStream_t)stream)));
+  TYLO_DISPATCH_DTYPE(dtype, T, return (M % Elem<T>::kVec ? softmax_launch<T, false, true>(dX, dY, Y, M, N, (cudaStream_t)stream)
+                                                       : softmax_launch<T, false, false>(dX, dY, Y, M, N, (cudaStream_t)stream)));
   return TYLO_OK;
 }
