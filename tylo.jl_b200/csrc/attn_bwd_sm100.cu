@@ -203,6 +203,7 @@ attn_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   // Ragged batches (attention.jl:25-26,60): keys at or beyond k_lengths[b] do not exist; 64-row query
   // blocks starting at or beyond q_lengths[b] were skipped by the forward and take no part here.
   int k_len = p.Sk, q_lim = p.Sq;
+  const bool trim = !ORS && (p.mask_flags & TYLO_MASK_DOCUMENT) && p.block_sparse;   // (every warp works it out for itself)
   auto batch_lengths = [&](int bb) {
     if (p.k_lengths) { const int v = p.k_lengths[bb]; k_len = v < 0 ? 0 : (v > p.Sk ? p.Sk : v); }
     if (p.q_lengths) {
@@ -221,6 +222,12 @@ attn_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     int lo = 0, hi = 0;
     if (own0 < k_len) q_range(p, own0, min(own0 + BT, k_len) - 1, q_lim, &lo, &hi);
     it_lo = lo / BT; it_n = hi > lo ? (hi - 1) / BT - it_lo + 1 : 0;
+    if (trim && it_n > 0) {
+      int t1 = it_lo + it_n;
+      doc_trim(p.doc_kv + (size_t)b * p.doc_stride + own0, min(own0 + BT, k_len) - own0,
+               p.doc_q + (size_t)b * p.doc_stride + p.input_pos, q_lim, it_lo, t1);
+      it_n = t1 - it_lo;
+    }
     n_iter = it_n * p.G;
   } else {
     const int nqt = (p.Sq + BT - 1) / BT;
@@ -230,6 +237,12 @@ attn_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     int lo = 0, hi = 0;
     if (own0 < q_lim) kv_range(p, own0 + p.input_pos, min(own0 + BT, q_lim) - 1 + p.input_pos, k_len, &lo, &hi);
     it_lo = lo / BT; it_n = hi > lo ? (hi - 1) / BT - it_lo + 1 : 0;
+    if (trim && it_n > 0) {
+      int t1 = it_lo + it_n;
+      doc_trim(p.doc_q + (size_t)b * p.doc_stride + own0 + p.input_pos, min(own0 + BT, q_lim) - own0,
+               p.doc_kv + (size_t)b * p.doc_stride, k_len, it_lo, t1);
+      it_n = t1 - it_lo;
+    }
     n_iter = it_n;
   }
 

@@ -171,9 +171,10 @@ __device__ __forceinline__ int fwd_slot_block(const FwdPlan& pl, int s, int e, i
 }
 
 // bm_t0 / bm_t1: with a host-built block list, the key tiles [t0, t1) that hold every listed block of the rows of
-// Q tile A and B (worked out by a whole warp, see the kernel); unused otherwise.
+// Q tile A and B (worked out by a whole warp, see the kernel); unused otherwise.  trim: called by a whole warp, drop key
+// tiles at either end that hold no document of the rows.
 __device__ __forceinline__ FwdItem fwd_item(const AttnParams& p, const FwdPlan& pl, uint32_t mask_flags, int hb, int qt,
-                                            const int* bm_t0 = nullptr, const int* bm_t1 = nullptr) {
+                                            const int* bm_t0, const int* bm_t1, const bool trim) {
   FwdItem it;
   const int hpb = p.H / pl.heads;
   it.b = hb / hpb; it.h = (hb % hpb) * pl.heads; it.hk = it.h / p.G; it.q0 = qt * pl.rows;
@@ -201,6 +202,13 @@ __device__ __forceinline__ FwdItem fwd_item(const AttnParams& p, const FwdPlan& 
       int lo, hi;
       kv_range(pr, qx + p.input_pos, min(qx + BM, p.Sq) - 1 + p.input_pos, it.k_len, &lo, &hi);
       if (hi > lo) { t0[X] = lo / BN; t1[X] = (hi - 1) / BN + 1; }
+      if (trim && hi > lo) {
+        if (X == 1 && pl.q_step == 0) { t0[1] = t0[0]; t1[1] = t1[0]; }      // the same rows
+        else
+          doc_trim(p.doc_q + (size_t)it.b * p.doc_stride + qx + p.input_pos, min(qx + BM, it.q_lim) - qx,
+                   p.doc_kv + (size_t)it.b * p.doc_stride, it.k_len, t0[X], t1[X]);
+        if (t1[X] <= t0[X]) { t0[X] = 0; t1[X] = 0; }
+      }
     }
   }
   const bool actA = t1[0] > t0[0], actB = t1[1] > t0[1];
@@ -816,8 +824,10 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         if (hi >= lo) { bm_t0[X] = lo * p.bm_tn / BN; bm_t1[X] = ((hi + 1) * p.bm_tn + BN - 1) / BN; }
       }
     }
-    // the item table: thread k of the two spare warps works out item k
-    const int k = threadIdx.x - 64;
+    // the item table: thread k of the two spare warps works out item k; with documents (one item per CTA) the whole first
+    // spare warp works out the one item
+    const bool trim = (mask_flags & TYLO_MASK_DOCUMENT) && p.block_sparse && p.n_or == 0 && !p.bm_count && n_local == 1;
+    const int k = trim ? warp - 2 : threadIdx.x - 64;
     if (k < n_local) {
       volatile int* e = tab + k * IT_WORDS;
       int hb;
@@ -826,7 +836,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       if (qt < 0) {
         e[IT_NTOT] = -1;                       // no such entry (middle block of an odd count)
       } else {
-        const FwdItem it = fwd_item(p, plan, mask_flags, hb, qt, bm_t0, bm_t1);
+        const FwdItem it = fwd_item(p, plan, mask_flags, hb, qt, bm_t0, bm_t1, trim);
 #pragma unroll
         for (int X = 0; X < 2; ++X) {
           volatile int* w = e + X * WI_WORDS;
@@ -984,6 +994,11 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
                 issue_qk(X, j + 1);
               }
             }
+            // a tile that neither Q tile takes part in (their ranges may leave a gap) has to have arrived all the same before
+            // its stage is handed back
+            if (ok && !v_ready) ok = mbar_wait(bar(SM::V_FULL + st), (gj / ST) & 1, abort_flag, &g_attn_fwd_status, 204);
+            if (ok && !k_ready && j + 1 < n_tot)
+              ok = mbar_wait(bar(SM::K_FULL + (gj + 1) % ST), ((gj + 1) / ST) & 1, abort_flag, &g_attn_fwd_status, 203);
             if (!ok) break;
             tc_commit(bar(SM::V_EMPTY + st));
             if (j + 1 < n_tot) {

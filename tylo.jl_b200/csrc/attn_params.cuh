@@ -139,4 +139,44 @@ __device__ __forceinline__ void q_range(const AttnParams& p, int kv_lo, int kv_h
   *lo = l; *hi = h;
 }
 
+// Narrows the 128-row tiles [t0, t1) of the streamed side (ids `str`, n_str rows) to those between the first and the last
+// that may share a document with the owned rows (ids `own`, n_own rows, at most 128): a tile whose span of ids does not meet
+// the span of the owned ids holds no unmasked pair, whatever the order of the ids.  Called by a whole warp.  A tile step of
+// the tensor-core kernels costs some 4,000 clocks with or without unmasked pairs; this costs one round trip to memory when
+// nothing can be dropped (owned ids, four tiles from the front and four from the back are asked for together) and one
+// more for every further four tiles that fall away.
+__device__ __forceinline__ void doc_trim(const int32_t* __restrict__ own, int n_own, const int32_t* __restrict__ str, int n_str,
+                                         int& t0, int& t1) {
+  const int lane = threadIdx.x & 31;
+  int o[4], f[4][4], k[4][4];
+  auto load = [&](int (&v)[4][4], int first, int step) {
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[t][i] = __ldg(str + min(min(max(first + t * step, t0), t1 - 1) * 128 + lane + 32 * i, n_str - 1));
+  };
+#pragma unroll
+  for (int i = 0; i < 4; ++i) o[i] = __ldg(own + min(lane + 32 * i, n_own - 1));
+  load(f, t0, 1);
+  load(k, t1 - 1, -1);
+  const int omin = __reduce_min_sync(0xffffffffu, min(min(o[0], o[1]), min(o[2], o[3])));
+  const int omax = __reduce_max_sync(0xffffffffu, max(max(o[0], o[1]), max(o[2], o[3])));
+  auto hits = [&](const int (&v)[4][4]) {
+    int bits = 0;
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      const int lo = __reduce_min_sync(0xffffffffu, min(min(v[t][0], v[t][1]), min(v[t][2], v[t][3])));
+      const int hi = __reduce_max_sync(0xffffffffu, max(max(v[t][0], v[t][1]), max(v[t][2], v[t][3])));
+      bits |= (lo <= omax && hi >= omin) << t;
+    }
+    return bits;
+  };
+  int fb = hits(f), kb = hits(k);
+  while (!fb && t0 + 4 < t1) { t0 += 4; load(f, t0, 1); fb = hits(f); }
+  if (!fb) { t1 = t0; return; }
+  t0 += __ffs(fb) - 1;
+  while (!kb) { t1 -= 4; load(k, t1 - 1, -1); kb = hits(k); }     // ends: tile t0 meets the owned ids
+  t1 -= __ffs(kb) - 1;
+}
+
 }  // namespace tylo
