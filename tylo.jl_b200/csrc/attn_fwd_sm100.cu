@@ -71,9 +71,10 @@ template <int DB> struct FwdSmem {
   static constexpr int kBars = kV + kStages * kTile;    // 8-byte mbarriers
   static constexpr int Q_FULL = 0, K_FULL = 2, K_EMPTY = K_FULL + kStages, V_FULL = K_EMPTY + kStages,
                        V_EMPTY = V_FULL + kStages, S_FULL = V_EMPTY + kStages, P_FULL = S_FULL + 2,
-                       O_READY = P_FULL + 2, Q_EMPTY = O_READY + 2, O_FREE = Q_EMPTY + 1, DONE = O_FREE + 2,
+                       P_TAIL = P_FULL + 2, O_READY = P_TAIL + 2, Q_EMPTY = O_READY + 2, O_FREE = Q_EMPTY + 1, DONE = O_FREE + 2,
                        kNumBars = DONE + 1;
   // Q_EMPTY: every Q K^T product of the finished work item has been issued, its Q tiles may be overwritten;
+  // P_FULL, P_TAIL: P of the first 96 keys / of the last 32 keys of a tile is in tensor memory (chunked form: P_FULL, all of it);
   // O_FREE: the softmax warpgroup has read the item's accumulator out of tensor memory (items in which its tile has keys).
   static constexpr int kMisc = kBars + 8 * kNumBars;    // tmem base, abort flag
   static constexpr int kItems = kMisc + 16;             // item table
@@ -128,6 +129,11 @@ __device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, uint32_t sr
 }
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+
+// The form of the tile loop (see softmax_tile).  In the register-resident form P is handed to the MMA issuer in two parts:
+// the product over the first 96 keys runs under the exponentials of the last 32, so that only a quarter of P V is left in
+// the chain softmax -> P V -> Q K^T of a Q tile (causal forward, S 4096, D 128: 488 -> 480 us).
+constexpr bool fwd_chunked(uint32_t mask, uint32_t score) { return (mask & ~(uint32_t)TYLO_MASK_CAUSAL) != 0 || score != 0; }
 
 struct TileRange { int s, e; };  // CTA-local key-tile indices [s, e) a Q tile takes part in
 
@@ -260,7 +266,7 @@ __device__ __forceinline__ bool softmax_tile(const AttnParams& p, const uint32_t
   // because the mod and mask code of a whole unrolled tile does not fit the instruction cache next to the other
   // roles (config-4 mods: 0.336 ms register-resident, 0.279 ms chunked; the plain causal forward is 7 % slower
   // chunked, since it reads every score twice for nothing).
-  constexpr bool kChunked = (MASK & ~(uint32_t)TYLO_MASK_CAUSAL) != 0 || SCORE != 0;
+  constexpr bool kChunked = fwd_chunked(MASK, SCORE);
   auto bar = [&](int i) { return sbase + SM::kBars + 8 * i; };
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int wq = warp & 3;                       // TMEM lane quarter this warp may touch
@@ -356,6 +362,7 @@ __device__ __forceinline__ bool softmax_tile(const AttnParams& p, const uint32_t
       tc_wait_st();
       tc_fence_before();
       mbar_arrive(bar(SM::P_FULL + X));
+      if (!kChunked) mbar_arrive(bar(SM::P_TAIL + X));
     };
     if (!listed_walk && (mask_flags & TYLO_MASK_DOCUMENT) && doc_uniform && __all_sync(0xffffffffu, ids[0] != my_doc)) {
       // all 128 keys belong to one document that none of this warp's 32 rows belongs to
@@ -634,7 +641,11 @@ __device__ __forceinline__ bool softmax_tile(const AttnParams& p, const uint32_t
       return s0 + s1;
     };
     if constexpr (!kChunked) {
-      const float s0 = exp_chunk(sr[0], 0), s1 = exp_chunk(sr[1], 1), s2 = exp_chunk(sr[2], 2), s3 = exp_chunk(sr[3], 3);
+      const float s0 = exp_chunk(sr[0], 0), s1 = exp_chunk(sr[1], 1), s2 = exp_chunk(sr[2], 2);
+      tc_wait_st();
+      tc_fence_before();
+      mbar_arrive(bar(SM::P_FULL + X));
+      const float s3 = exp_chunk(sr[3], 3);
       l += (s0 + s1) + (s2 + s3);
     } else {
       // Pass 2: P chunk q lands on the columns of score chunk q / 2, which has been read by then.
@@ -657,7 +668,7 @@ __device__ __forceinline__ bool softmax_tile(const AttnParams& p, const uint32_t
     }
     tc_wait_st();
     tc_fence_before();
-    mbar_arrive(bar(SM::P_FULL + X));
+    mbar_arrive(bar((kChunked ? SM::P_FULL : SM::P_TAIL) + X));
   }
 
   // ---- epilogue: O / l, M, L   (tcgen05.ld is warp-collective: every lane loads, stores are predicated)
@@ -788,7 +799,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       mbar_init(bar(SM::V_FULL + s), 1); mbar_init(bar(SM::V_EMPTY + s), 1);
     }
     for (int i = 0; i < 2; ++i) {
-      mbar_init(bar(SM::S_FULL + i), 1); mbar_init(bar(SM::P_FULL + i), 128); mbar_init(bar(SM::O_READY + i), 1);
+      mbar_init(bar(SM::S_FULL + i), 1); mbar_init(bar(SM::P_FULL + i), 128); mbar_init(bar(SM::P_TAIL + i), 128); mbar_init(bar(SM::O_READY + i), 1);
       mbar_init(bar(SM::O_FREE + i), 128);
     }
     mbar_init(bar(SM::Q_EMPTY), 1);
@@ -955,9 +966,15 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             const uint64_t vd = desc_at(dv_hi, sbase + SM::kV + ((g0 + j) % ST) * SM::kTile);
             const bool first = (j == ts[X]);
 #pragma unroll
-            for (int kk = 0; kk < BN / kKeysPerMma; ++kk)     // 8 columns of P and kKeysPerMma rows of V per step
+            for (int kk = 0; kk < BN / kKeysPerMma; ++kk) {   // 8 columns of P and kKeysPerMma rows of V per step
+              if (!fwd_chunked(MASK, SCORE) && kk == BN / kKeysPerMma * 3 / 4) {
+                ok = mbar_wait(bar(SM::P_TAIL + X), (cb[X] + j - ts[X]) & 1, abort_flag, &g_attn_fwd_status, 207);
+                if (!ok) break;
+                tc_fence_after();
+              }
               mma_ts<kTf32>(tmem + 256 + X * 128, pa + kk * 8, vd + (uint32_t)((kk * kKeysPerMma * 128) >> 4), idesc_pv,
                             !first || (kk > 0));
+            }
             tc_commit(bar(SM::O_READY + X));
           };
           ok = mbar_wait(bar(SM::Q_FULL + 0), ni & 1, abort_flag, &g_attn_fwd_status, 201);
