@@ -196,7 +196,8 @@ __device__ __forceinline__ void decode_tail(const DecodeTail& tail, float* Op, f
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  if (gsz > 1) {
+  // (with a single group its last CTA goes on to the final merge, over the splits themselves: no fold, no second ticket)
+  if (gsz > 1 && n_groups > 1) {
     for (int g = warp; g < G; g += NWARPS) {
       const size_t hb = (size_t)b * H + (size_t)hk * G + g;
       float o[D / 32], m, l;
@@ -209,16 +210,19 @@ __device__ __forceinline__ void decode_tail(const DecodeTail& tail, float* Op, f
   }
 
   // ---- level 2: the CTA that completes the last group merges the group partials -----------------------
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const int t = atomicAdd(&tk[n_groups], 1);
-    s_last = (t == n_groups - 1);
-    if (s_last) tk[n_groups] = 0;
+  if (n_groups > 1) {
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      const int t = atomicAdd(&tk[n_groups], 1);
+      s_last = (t == n_groups - 1);
+      if (s_last) tk[n_groups] = 0;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
   }
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
+  const int step = n_groups > 1 ? kGroup : 1, count = n_groups > 1 ? n_groups : gsz;
   T* O = static_cast<T*>(tail.O);
   const int world = tail.world, rank = tail.rank;
   const ExchangeLayout lay = exchange_layout(world, (int)BH, D);
@@ -233,7 +237,7 @@ __device__ __forceinline__ void decode_tail(const DecodeTail& tail, float* Op, f
     const int g = warp + k * NWARPS;
     if (g >= G) break;
     const size_t hb = (size_t)b * H + (size_t)hk * G + g;
-    merge_slots<D>(Op, Mp, Lp, BH, hb, 0, kGroup, n_groups, lane, o[k], m[k], l[k]);
+    merge_slots<D>(Op, Mp, Lp, BH, hb, 0, step, count, lane, o[k], m[k], l[k]);
     if (world > 1) {
       epoch[k] = self[lay.epoch_off + hb] + 1u;     // call counter of this head
       const int par = (int)(epoch[k] & 1u);
