@@ -106,25 +106,19 @@ __device__ __forceinline__ float ex2_fast(float x) {
 // registers of an fp32 copy, so twice the bytes in flight per SM for the same occupancy) and exp is
 // evaluated twice per element (once for the sum, once for the output) on the otherwise idle
 // special-function unit; its approximate form is ample for a 16-bit result.
-// (at 16 packets per thread three CTAs per SM are asked for: 80 registers; left alone the compiler takes 128, and 2048 rows
-// of 32,768 bf16 go from 51 to 57 us)
+// (ragged rows at 16 packets per thread: left alone the compiler takes 226 registers; three CTAs per SM are asked for)
 template <typename T, int THREADS, int ITERS, bool RAGGED>
-__global__ void __launch_bounds__(row_cta(THREADS), ITERS == 16 ? 3 : 1)
+__global__ void __launch_bounds__(row_cta(THREADS), RAGGED && ITERS == 16 ? 3 : 0)
 softmax_fwd_packed_kernel(T* __restrict__ Y, const T* __restrict__ X, int64_t M, int N) {
   constexpr int VEC = Elem<T>::kVec;
   __shared__ float smem[32];
-  int nvec = (int)(M / VEC);
   const size_t row = row_index<THREADS>();
   if (THREADS == 32 && row >= (size_t)N) return;
   const int tid = row_thread<THREADS>();
+  const int nvec = RAGGED ? RaggedRow<T>(X + row * M, M).nvec : (int)(M / VEC);
   RowRegs<T, THREADS, ITERS> r;
-  if constexpr (RAGGED) {
-    const RaggedRow<T> x(X + row * M, M);
-    nvec = (int)x.nvec;
-    r.load(x, -INFINITY);
-  } else {
-    r.load(X + row * M, nvec);
-  }
+  if constexpr (RAGGED) r.load(RaggedRow<T>(X + row * M, M), -INFINITY);
+  else r.load(X + row * M, nvec);
   float m = -INFINITY;
 #pragma unroll
   for (int i = 0; i < ITERS; ++i) {
