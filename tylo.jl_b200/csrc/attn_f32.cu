@@ -10,6 +10,11 @@
 // the streamed tiles in turn, each with its own tiles, statistics and accumulators, and are merged once at the end: small
 // problems have about one CTA per SM, and one group's loads and exponentials run under the other groups' FMAs.
 //
+// Packed pairs (fma.rn.f32x2) are used where their accumulators fit: they take half the issue slots, and with more warps
+// than the registers allow here twice the rate.  Measured, forward + backward: B2 H8 S512 D64 825 us on the 2 x 2 patches,
+// 209 with 4 x 8 patches, 204 with 8 x 8, 197 with packed pairs; the FMA pipes are 46 % / 40 % busy (forward / backward), eight
+// warps per SM do not hide the shared-memory latency.
+//
 // Forward: online softmax per group.  Backward: no atomics on dQ / dK / dV; dK / dV CTAs (own 64 keys, sum the query heads
 // of the group) and dQ CTAs (own 64 queries) share one launch, heaviest first, so that both fill the SMs together.
 #include "attn_dispatch.cuh"

@@ -1,8 +1,9 @@
 // Shape- and dtype-generic attention forward / backward in fp32 arithmetic (CUDA cores).
 //
-// This path serves (a) fp32 storage, where the contract is true-fp32 accuracy (the reference's
-// default rounds fp32 operands to TF32, utils.jl:40-44), and (b) every shape or mod combination
-// the tcgen05 kernels do not cover (head dims other than 64/128, ragged per-batch lengths, ...).
+// This path serves every shape or mod combination that neither the tcgen05 kernels nor the fp32 kernels of attn_f32.cu
+// cover: head dims above 128, that are not multiples of 8 (4 in fp32) or with Dk != Dv, OR-ed clauses with a document
+// term, block lists in the backward and in fp32.  fp32 storage means true-fp32 accuracy here as there (the reference's
+// default rounds fp32 operands to TF32, utils.jl:40-44).
 // It is written for correctness and reasonable speed, not for the roofline: 32x32 tiles staged
 // in shared memory as fp32, 256 threads, each owning a 2x2 patch of the score tile and a
 // 2 x (D/16) patch of the output tile.
