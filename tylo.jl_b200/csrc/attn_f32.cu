@@ -12,7 +12,7 @@
 //
 // Packed pairs (fma.rn.f32x2) are used where their accumulators fit: they take half the issue slots, and with more warps
 // than the registers allow here twice the rate.  Measured, forward + backward: B2 H8 S512 D64 825 us on the 2 x 2 patches,
-// 209 with 4 x 8 patches, 204 with 8 x 8, 197 with packed pairs; the FMA pipes are 46 % / 40 % busy (forward / backward), eight
+// 209 with 4 x 8 patches, 204 with 8 x 8, 197 with packed pairs, 201 with short chains; the FMA pipes are 46 % / 40 % busy (forward / backward), eight
 // warps per SM do not hide the shared-memory latency.
 //
 // Forward: online softmax per group.  Backward: no atomics on dQ / dK / dV; dK / dV CTAs (own 64 keys, sum the query heads
@@ -98,7 +98,7 @@ __device__ __forceinline__ void dot_tile(const float* __restrict__ X, const floa
       const float4 b = *reinterpret_cast<const float4*>(y + j * TX * (D + 4) + c);
 #pragma unroll
       for (int i = 0; i < RT; ++i)
-        out[i][j] = fmaf(a[i].w, b.w, fmaf(a[i].z, b.z, fmaf(a[i].y, b.y, fmaf(a[i].x, b.x, out[i][j]))));
+        out[i][j] += fmaf(a[i].w, b.w, fmaf(a[i].z, b.z, fmaf(a[i].y, b.y, a[i].x * b.x)));      // (short chains: D / 4 sums)
     }
   }
 }
@@ -387,20 +387,15 @@ __device__ __forceinline__ void bwd_tiles(float* sm, float* __restrict__ dA, flo
     kv_range(p, own0 + p.input_pos, min(own0 + BR, q_lim) - 1 + p.input_pos, k_len, &lo, &hi);
   }
   const int t0 = lo / SB, nt = hi > lo ? (hi - 1) / SB + 1 - t0 : 0;
-  const int n_iter = OWN_KEYS ? nt * p.G : nt;
 
   uint64_t acc1[RT][OC / 2], acc2[RT][OC / 2];        // (acc1: dV, OWN_KEYS only)
-#pragma unroll
-  for (int i = 0; i < RT; ++i)
-#pragma unroll
-    for (int e = 0; e < OC / 2; ++e) { acc1[i][e] = 0ull; acc2[i][e] = 0ull; }
   float slope_acc = 0.f;
 
-  // (Y1, Y2) of streamed tile n: queries and their dO of head h0 + n / nt, or keys and values
-  auto load_y = [&](int n) {
-    const int row0 = (t0 + (OWN_KEYS ? n % nt : n)) * SB;
+  // (Y1, Y2) of streamed tile n: queries and their dO of query head h, or keys and values
+  auto load_y = [&](int n, int h) {
+    const int row0 = (t0 + n) * SB;
     if (OWN_KEYS) {
-      const size_t hq = (size_t)(b * p.H + h0 + n / nt) * p.Sq;
+      const size_t hq = (size_t)(b * p.H + h) * p.Sq;
       load_tile<D, SB, GT>(sY1, Q + hq * p.Dk, row0, q_lim, p.Dk, tid);
       load_tile<D, SB, GT>(sY2, dO + hq * p.Dk, row0, q_lim, p.Dk, tid);
       if (tid < SB) {
@@ -414,7 +409,7 @@ __device__ __forceinline__ void bwd_tiles(float* sm, float* __restrict__ dA, flo
     }
   };
 
-  if (n_iter > 0) {
+  if (nt > 0) {
     if (OWN_KEYS) {
       load_tile<D, BR, kThreads>(sX1, Kg, own0, k_len, p.Dk, threadIdx.x);
       load_tile<D, BR, kThreads>(sX2, Vg, own0, k_len, p.Dk, threadIdx.x);
@@ -432,11 +427,18 @@ __device__ __forceinline__ void bwd_tiles(float* sm, float* __restrict__ dA, flo
   cp_commit();
   cp_wait<0>();
   __syncthreads();
-  for (int n = grp; n < n_iter; n += NG) {
-    const int str0 = (t0 + (OWN_KEYS ? n % nt : n)) * SB;
-    const int h = OWN_KEYS ? h0 + n / nt : h0;
+  // dK / dV: one query head of the group at a time, summed into the outputs head by head, so that an accumulator's chain is no
+  // longer than a head's share of rows
+  for (int g = 0; g < (OWN_KEYS ? p.G : 1); ++g) {
+  const int h = h0 + g;
+#pragma unroll
+  for (int i = 0; i < RT; ++i)
+#pragma unroll
+    for (int e = 0; e < OC / 2; ++e) { acc1[i][e] = 0ull; acc2[i][e] = 0ull; }
+  for (int n = grp; n < nt; n += NG) {
+    const int str0 = (t0 + n) * SB;
     sh.sync();                  // everyone is done with the tile before
-    load_y(n);
+    load_y(n, h);
     cp_commit();
     cp_wait<0>();
     sh.sync();
@@ -535,15 +537,21 @@ __device__ __forceinline__ void bwd_tiles(float* sm, float* __restrict__ dA, flo
       if (row >= S) break;
       float4 t = *reinterpret_cast<const float4*>(gs + r * (D + 4) + col);
 #pragma unroll
-      for (int g = 1; g < NG; ++g) {
-        const float4 x = *reinterpret_cast<const float4*>(gs + g * SM::kGroup + r * (D + 4) + col);
+      for (int k = 1; k < NG; ++k) {
+        const float4 x = *reinterpret_cast<const float4*>(gs + k * SM::kGroup + r * (D + 4) + col);
         t.x += x.x; t.y += x.y; t.z += x.z; t.w += x.w;
       }
-      if (col < p.Dk) *reinterpret_cast<float4*>(out + (base + row) * p.Dk + col) = t;
+      if (col < p.Dk) {
+        float4* o = reinterpret_cast<float4*>(out + (base + row) * p.Dk + col);
+        if (g > 0) { const float4 q = *o; t.x += q.x; t.y += q.y; t.z += q.z; t.w += q.w; }     // (this thread's own earlier store)
+        *o = t;
+      }
     }
   };
   if constexpr (OWN_KEYS) merge(acc1, dB);
   merge(acc2, dA);
+  __syncthreads();              // the groups' tiles have been read
+  }
   if (!OWN_KEYS && p.d_slopes && (p.score_flags & TYLO_SCORE_ALIBI)) {
     slope_acc = warp_reduce(slope_acc, SumOp());
     if (sh.lane == 0 && slope_acc != 0.f) atomicAdd(p.d_slopes + h0, slope_acc);
