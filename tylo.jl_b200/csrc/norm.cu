@@ -661,9 +661,10 @@ norm_bwd_reduce_kernel(T* __restrict__ dW, T* __restrict__ dB, const float* __re
 // ------------------------------------------------------------------------------------------------
 // host side
 // ------------------------------------------------------------------------------------------------
-// Shared memory beyond 48 KB has to be asked for; below that the call would only cost the host time.
+// More than 48 KB of shared memory has to be asked for; below that the call would only cost the host time.  The 48 KB hold a
+// kernel's static arrays too, so the line for the dynamic part lies 1 KB lower (the kernels here have at most 256 bytes of them).
 template <typename K> static int32_t allow_smem(K kern, int64_t bytes) {
-  if (bytes > 48 * 1024) TYLO_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  if (bytes > 47 * 1024) TYLO_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
   return TYLO_OK;
 }
 
