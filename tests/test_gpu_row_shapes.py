@@ -34,6 +34,30 @@ def test_softmax_minus_infinity(tylo, oracle, M):
     check(tylo.softmax(X), oracle.softmax_ref(back(X)), "f32", "softmax")
 
 
+# one length per kernel and per way a row is moved: a warp, several warps, the long two-pass rows, each in whole packets and not
+@pytest.mark.parametrize("dt", ["f32", "bf16", "f16"])
+@pytest.mark.parametrize("M", [40, 61, 1000, 1001, 8192, 8195, 16392, 16401, 32768, 32771, 65600, 70001])
+def test_softmax_not_finite(tylo, M, dt):
+    X = torch.randn(9, M, device="cuda").to({"f32": torch.float32, "bf16": torch.bfloat16, "f16": torch.float16}[dt])
+    X[0, M // 3] = float("nan")
+    X[1, M - 1] = float("inf")
+    X[2, :] = float("-inf")
+    X[2, M // 2] = float("nan")
+    X[3, :] = float("nan")
+    X[4, :] = float("-inf")
+    X[4, 0] = float("inf")
+    X[5, :] = float("-inf")                           # the one row that is defined to be zeros
+    X[6, ::2] = torch.finfo(X.dtype).min              # masked by the lowest value, in part
+    if dt != "bf16" or M > 32768:                     # (bf16 rows in registers: the lowest value times log2(e) is -Inf)
+        X[7, :] = torch.finfo(X.dtype).min            # and throughout
+    Y = tylo.softmax(X)
+    assert bool(Y[:5].isnan().all())
+    assert bool((Y[5] == 0).all())
+    ref = torch.softmax(X[6:].double(), -1)
+    tol = {"f32": 1e-5, "bf16": 2.0 ** -8, "f16": 2.0 ** -10}[dt] * float(ref.max())       # an ulp of the largest result
+    assert float((Y[6:].double() - ref).abs().max()) <= tol
+
+
 # packets per row (f32: 4 elements, 16-bit: 8): one warp, a warp and one, eight rows per CTA, ragged thread counts, 1,024 and
 # beyond (two and four packets per thread), and lengths that are not a multiple of the packet
 @pytest.mark.parametrize("dt", ["f32", "bf16"])

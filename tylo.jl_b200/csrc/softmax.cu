@@ -14,7 +14,10 @@ namespace tylo {
 
 constexpr float kLog2e = 1.4426950408889634f;
 
-// Combine a per-thread (max, sum-relative-to-that-max) pair over the row's threads.  Returns the row max and the row sum relative to it.
+// Combine a per-thread (max, sum-relative-to-that-max) pair over the row's threads.  Returns the row max and the row sum relative
+// to it; the sum is 0 for a row made only of -Inf and NaN for a row that holds a NaN or +Inf, wherever in it (fmaxf passes over
+// a NaN, so a part of -Inf and NaN has maximum -Inf and a NaN as its sum).  Differences are taken before the factor log2(e): the
+// lowest finite fp32 value would overflow with it.
 template <int THREADS>
 __device__ __forceinline__ void reduce_max_sum(float& m, float& s, float* smem /* >= 64 floats */) {
   // warp level
@@ -22,7 +25,7 @@ __device__ __forceinline__ void reduce_max_sum(float& m, float& s, float* smem /
   for (int o = 16; o > 0; o >>= 1) {
     const float m2 = __shfl_xor_sync(0xffffffffu, m, o), s2 = __shfl_xor_sync(0xffffffffu, s, o);
     const float mn = fmaxf(m, m2);
-    s = (mn == -INFINITY) ? 0.f : s * exp2f(m - mn) + s2 * exp2f(m2 - mn);
+    s = (mn == -INFINITY) ? s + s2 : s * exp2f((m - mn) * kLog2e) + s2 * exp2f((m2 - mn) * kLog2e);
     m = mn;
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -35,7 +38,7 @@ __device__ __forceinline__ void reduce_max_sum(float& m, float& s, float* smem /
     for (int o = 16; o > 0; o >>= 1) {
       const float m2 = __shfl_xor_sync(0xffffffffu, m, o), s2 = __shfl_xor_sync(0xffffffffu, s, o);
       const float mn = fmaxf(m, m2);
-      s = (mn == -INFINITY) ? 0.f : s * exp2f(m - mn) + s2 * exp2f(m2 - mn);
+      s = (mn == -INFINITY) ? s + s2 : s * exp2f((m - mn) * kLog2e) + s2 * exp2f((m2 - mn) * kLog2e);
       m = mn;
     }
   }
@@ -82,10 +85,9 @@ softmax_fwd_kernel(T* __restrict__ Y, const T* __restrict__ X, int64_t M, int N)
       s += e[i][j];
     }
   }
-  m *= kLog2e;  // reductions run in log2 units
   reduce_max_sum<THREADS>(m, s, smem);
-  // a row made only of -Inf yields zeros (nothing in the reference's tests pins that case)
-  const float factor = (m_thread == -INFINITY) ? 0.f : exp2f(m_thread * kLog2e - m) / s;
+  // a row made only of -Inf yields zeros (nothing in the reference's tests pins that case); a NaN sum reaches every element
+  const float factor = s == 0.f ? 0.f : ((m_thread == -INFINITY) ? 0.f : exp2f((m_thread - m) * kLog2e)) / s;
 #pragma unroll
   for (int i = 0; i < ITERS; ++i) {
 #pragma unroll
@@ -140,7 +142,7 @@ softmax_fwd_packed_kernel(T* __restrict__ Y, const T* __restrict__ X, int64_t M,
     }
   }
   s = block_reduce<THREADS>(s, SumOp(), 0.f, smem);
-  const float inv = s > 0.f ? 1.f / s : 0.f;
+  const float inv = (m == -INFINITY && s == 0.f) ? 0.f : 1.f / s;     // only -Inf: zeros; NaN or +Inf in the row: NaN throughout
 #pragma unroll
   for (int i = 0; i < ITERS; ++i) {
     float f[VEC]; r.p[i].unpack(f);
@@ -173,7 +175,7 @@ softmax_fwd_twopass_kernel(T* __restrict__ Y, const T* __restrict__ X, int64_t M
     p.pack(f);
     return p;
   };
-  float m = -INFINITY, s = 0.f;        // m in log2 units
+  float m = -INFINITY, s = 0.f;
   for (int v0 = threadIdx.x; v0 < nvec; v0 += U * THREADS) {
     Pack<T> p[U];
 #pragma unroll
@@ -185,9 +187,9 @@ softmax_fwd_twopass_kernel(T* __restrict__ Y, const T* __restrict__ X, int64_t M
 #pragma unroll
       for (int j = 0; j < VEC; ++j) mx = fmaxf(mx, f[j]);
     }
-    const float mn = fmaxf(m, mx * kLog2e);
+    const float mn = fmaxf(m, mx);
     if (mn != -INFINITY) {
-      s *= ex2(m - mn);
+      s *= ex2((m - mn) * kLog2e);
       m = mn;
     }
     const float mo = m == -INFINITY ? 0.f : m;
@@ -195,11 +197,11 @@ softmax_fwd_twopass_kernel(T* __restrict__ Y, const T* __restrict__ X, int64_t M
     for (int u = 0; u < U; ++u) {
       float f[VEC]; p[u].unpack(f);
 #pragma unroll
-      for (int j = 0; j < VEC; ++j) s += ex2(fmaf(f[j], kLog2e, -mo));
+      for (int j = 0; j < VEC; ++j) s += ex2((f[j] - mo) * kLog2e);
     }
   }
   reduce_max_sum<THREADS>(m, s, smem);
-  const float inv = m == -INFINITY ? 0.f : 1.f / s, mo = m == -INFINITY ? 0.f : m;
+  const float inv = s == 0.f ? 0.f : 1.f / s, mo = m == -INFINITY ? 0.f : m;
   for (int v0 = threadIdx.x; v0 < nvec; v0 += U * THREADS) {
     Pack<T> p[U];
 #pragma unroll
@@ -209,7 +211,7 @@ softmax_fwd_twopass_kernel(T* __restrict__ Y, const T* __restrict__ X, int64_t M
       const int v = v0 + u * THREADS;
       float f[VEC]; p[u].unpack(f);
 #pragma unroll
-      for (int j = 0; j < VEC; ++j) f[j] = ex2(fmaf(f[j], kLog2e, -mo)) * inv;
+      for (int j = 0; j < VEC; ++j) f[j] = ex2((f[j] - mo) * kLog2e) * inv;
       p[u].pack(f);
       if constexpr (RAGGED) y.store(v, p[u]);
       else if (v < nvec) st_stream(Y + base + (size_t)v * VEC, p[u].raw);
