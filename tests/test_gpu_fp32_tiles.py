@@ -1,9 +1,11 @@
-"""GPU parity: the register-tiled fp32 attention kernels at the edges of their 64-row tiles, their two groups of streamed
-tiles (an odd number of them, fewer than two), padded head dims (32 / 64 / 128)."""
+"""GPU parity: the register-tiled fp32 attention kernels at the edges of their 64-row tiles, of their groups of streamed
+tiles (four at head dims up to 64, two above: a number of tiles that is no multiple of them, fewer than them), of padded head
+dims (32 / 64 / 128), and on both sides of the lines to the general kernels (32 and 64 keys)."""
 import numpy as np
 import pytest
+import torch
 
-from gpu_util import check, draw
+from gpu_util import back, check, draw
 
 pytestmark = pytest.mark.gpu
 
@@ -23,4 +25,46 @@ def test_tiles(tylo, oracle, B, H, Hkv, Sq, Sk, pos, D, causal):
     check(O, oracle.flex_ref(Q64, K64, V64, **okw), "f32", "O")
     got = tylo.grad_flex_attention(dO, Q, K, V, O, checkpoints=cp, mask_mod=mask, input_pos=pos)
     for g, ref, name in zip(got, oracle.flex_bwd_ref(dO64, Q64, K64, V64, **okw), ("dQ", "dK", "dV")):
+        check(g, ref, "f32", name)
+
+
+def _mask(name, t, o, n):
+    ids = (np.arange(n) * 5 // n).astype(np.int32)
+    docs = t.DocumentMask(torch.from_numpy(ids).cuda())
+    if name == "causal & window & document":
+        return t.CausalMask() & t.SlidingWindowMask(20) & docs, o.MaskSpec(causal=True, window=20, doc_q=ids)
+    if name == "prefix & document":
+        return t.PrefixMask(37) & docs, o.MaskSpec(prefix=37, doc_q=ids)
+    if name == "prefix_lm":
+        return t.prefix_lm(19), o.MaskSpec(prefix_or_causal=19)
+    if name == "window | document":
+        return t.SlidingWindowMask(9) | docs, o.MaskAny(o.MaskSpec(window=9), o.MaskSpec(doc_q=ids))
+    return None, None
+
+
+# every mask term as the bits of a column of pairs, from the queries' side and from the keys', with each order of the score mods
+@pytest.mark.parametrize("mask", ["none", "causal & window & document", "prefix & document", "prefix_lm", "window | document"])
+@pytest.mark.parametrize("score", ["none", "alibi, then soft cap", "soft cap, then alibi", "bias, then soft cap"])
+@pytest.mark.parametrize("B,H,Hkv,Sq,Sk,D", [(1, 2, 1, 32, 32, 64), (1, 2, 2, 33, 33, 32), (2, 4, 2, 64, 64, 64), (40, 8, 8, 20, 30, 32),
+                                             (1, 2, 1, 65, 130, 128), (2, 3, 1, 150, 100, 36)])
+def test_masks_and_mods(tylo, oracle, B, H, Hkv, Sq, Sk, D, score, mask):
+    t, o = tylo, oracle
+    rng = np.random.default_rng(Sq + Sk + D)
+    Q, Q64 = draw(rng, (B, H, Sq, D), "f32"); K, K64 = draw(rng, (B, Hkv, Sk, D), "f32"); V, V64 = draw(rng, (B, Hkv, Sk, D), "f32")
+    dO, dO64 = draw(rng, (B, H, Sq, D), "f32")
+    m, om = _mask(mask, t, o, max(Sq, Sk))
+    slopes = torch.tensor([0.25 * 2.0 ** -h for h in range(H)], device="cuda")
+    table, table64 = draw(rng, (1, H, Sq, Sk), "f32")
+    alibi = (t.AliBiScore(slopes), ("alibi", back(slopes)))
+    cap = (t.SoftCapScore(3.0), ("softcap", 3.0))
+    chain = {"none": [], "alibi, then soft cap": [alibi, cap], "soft cap, then alibi": [cap, alibi],
+             "bias, then soft cap": [(t.BiasScore(table), ("bias", table64)), cap]}[score]
+    sm = chain[1][0] @ chain[0][0] if chain else None
+    kw = dict(mask_mod=m, score_mod=sm)
+    okw = dict(mask=om, score=o.ScoreSpec([c[1] for c in chain]) if chain else None)
+    cp = t.allocate_checkpoints_flex_attention(Q, K, V)
+    O = t.flex_attention(Q, K, V, checkpoints=cp, **kw)
+    check(O, o.flex_ref(Q64, K64, V64, **okw), "f32", "O")
+    got = t.grad_flex_attention(dO, Q, K, V, O, checkpoints=cp, **kw)
+    for g, ref, name in zip(got, o.flex_bwd_ref(dO64, Q64, K64, V64, **okw), ("dQ", "dK", "dV")):
         check(g, ref, "f32", name)

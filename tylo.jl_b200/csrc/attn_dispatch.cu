@@ -21,7 +21,7 @@ int32_t attn_fwd_dispatch(void* O, const void* Q, const void* K, const void* V, 
                           const AttnParams& p, int32_t dtype, cudaStream_t st) {
   if (!fwd_needs_generic(p) && attn_fwd_sm100_supported(p, dtype)) return attn_fwd_sm100(O, Q, K, V, M, L, p, dtype, st);
   if (dtype == TYLO_F32_TF32) dtype = TYLO_F32;      // no tensor-core form for this call: true fp32
-  if (attn_f32_supported(p, dtype)) return attn_fwd_f32(O, Q, K, V, M, L, p, st);
+  if (attn_fwd_f32_preferred(p, dtype)) return attn_fwd_f32(O, Q, K, V, M, L, p, st);
   TYLO_DISPATCH_DTYPE(dtype, T, return attn_fwd_generic<T>(O, Q, K, V, M, L, p, st));
   return TYLO_OK;
 }
@@ -39,7 +39,7 @@ int32_t attn_bwd_dispatch(void* dQ, void* dK, void* dV, const void* Q, const voi
                           void* workspace, const AttnParams& p, int32_t dtype, cudaStream_t st) {
   if (!table_mods(p) && attn_bwd_sm100_supported(p, dtype))
     return attn_bwd_sm100(dQ, dK, dV, Q, K, V, O, dO, M, L, Delta, workspace, p, dtype, st);
-  if (attn_f32_supported(p, dtype)) return attn_bwd_f32(dQ, dK, dV, Q, K, V, O, dO, M, L, Delta, p, st);
+  if (attn_bwd_f32_preferred(p, dtype)) return attn_bwd_f32(dQ, dK, dV, Q, K, V, O, dO, M, L, Delta, p, st);
   TYLO_DISPATCH_DTYPE(dtype, T, return attn_bwd_generic<T>(dQ, dK, dV, Q, K, V, O, dO, M, L, Delta, p, st));
   return TYLO_OK;
 }

@@ -13,8 +13,9 @@ int32_t attn_bwd_generic(void* dQ, void* dK, void* dV, const void* Q, const void
                          const void* O, const void* dO, const float* M, const float* L, float* Delta,
                          const AttnParams& p, cudaStream_t st);
 
-// register-tiled fp32 kernels (attn_f32.cu)
-bool attn_f32_supported(const AttnParams& p, int32_t dtype);
+// register-tiled fp32 kernels (attn_f32.cu); `preferred`: they cover the problem and beat the general kernels on it
+bool attn_fwd_f32_preferred(const AttnParams& p, int32_t dtype);
+bool attn_bwd_f32_preferred(const AttnParams& p, int32_t dtype);
 int32_t attn_fwd_f32(void* O, const void* Q, const void* K, const void* V, float* M, float* L, const AttnParams& p, cudaStream_t st);
 int32_t attn_bwd_f32(void* dQ, void* dK, void* dV, const void* Q, const void* K, const void* V, const void* O, const void* dO,
                      const float* M, const float* L, float* Delta, const AttnParams& p, cudaStream_t st);

@@ -135,6 +135,15 @@ __device__ __forceinline__ void put_transposed(float* U, int ty, int tx, const f
     u[1] = make_float4(v[4][j], v[5][j], v[6][j], v[7][j]);
   }
 }
+template <int D, int NJ>
+__device__ __forceinline__ void get_transposed(const float* U, int ty, int tx, float (&v)[RT][NJ]) {
+#pragma unroll
+  for (int j = 0; j < NJ; ++j) {
+    const float4* u = reinterpret_cast<const float4*>(U + (tx + Shape<D>::TX * j) * LDU + RT * ty);
+    const float4 a = u[0], b = u[1];
+    v[0][j] = a.x; v[1][j] = a.y; v[2][j] = a.z; v[3][j] = a.w; v[4][j] = b.x; v[5][j] = b.y; v[6][j] = b.z; v[7][j] = b.w;
+  }
+}
 // a thread's output patch to / from a BR x D tile in shared memory (row pitch D + 4)
 template <int D>
 __device__ __forceinline__ void put_rows(float* dst, int ty, int tx, const uint64_t (&a)[RT][Shape<D>::OC / 2]) {
@@ -161,6 +170,91 @@ __device__ __forceinline__ bool needs_mask(const AttnParams& p, int q0, int kv0,
   if (p.n_or > 0 || (p.mask_flags & ~(uint32_t)TYLO_MASK_CAUSAL)) return true;
   return (p.mask_flags & TYLO_MASK_CAUSAL) && kv0 + keys - 1 > q0 + p.input_pos;
 }
+__device__ __forceinline__ uint32_t low_bits(int n) { return (1u << max(0, min(n, RT))) - 1u; }
+// Which of the pairs (q + i, kv), or (q, kv + i) with OWN_KEYS, that are set in `live` a clause keeps: mask_keep for the RT own
+// rows of a column at once.  Every term but the documents is an interval of i, so a column costs a few instructions instead of a
+// few per pair; pairs that are not live are not looked up in the id tables.
+template <bool OWN_KEYS>
+__device__ __forceinline__ uint32_t clause_bits(uint32_t live, uint32_t flags, int window, int prefix_len, const int32_t* doc_q,
+                                                const int32_t* doc_kv, long long doc_stride, int b, int q, int kv) {
+  constexpr uint32_t kAll = (1u << RT) - 1u;
+  const int d = q - kv, w = min(window, 1 << 30);                                   // (positions are far below 2^30)
+  const uint32_t past = OWN_KEYS ? low_bits(d + 1) : kAll & ~low_bits(-d);          // query position >= key position
+  const uint32_t prefix = OWN_KEYS ? low_bits(prefix_len - kv) : (kv < prefix_len ? kAll : 0u);
+  if (flags & (TYLO_MASK_CAUSAL | TYLO_MASK_SLIDING)) live &= past;
+  if (flags & TYLO_MASK_SLIDING) live &= OWN_KEYS ? kAll & ~low_bits(d - w) : low_bits(w - d + 1);
+  if (flags & TYLO_MASK_PREFIX) live &= prefix;
+  if (flags & TYLO_MASK_PREFIX_LM) live &= past | prefix;
+  if ((flags & TYLO_MASK_DOCUMENT) && live) {
+    const int32_t* own = (OWN_KEYS ? doc_kv + kv : doc_q + q) + (size_t)b * doc_stride;
+    const int id = OWN_KEYS ? doc_q[(size_t)b * doc_stride + q] : doc_kv[(size_t)b * doc_stride + kv];
+    int ids[RT];
+#pragma unroll
+    for (int i = 0; i < RT; ++i) ids[i] = (live >> i) & 1u ? own[i] : id;
+#pragma unroll
+    for (int i = 0; i < RT; ++i) live &= ~((ids[i] != id ? 1u : 0u) << i);
+  }
+  return live;
+}
+// Bit 8 j + i: pair (i, j) of a thread's patch takes part.  own0: first own row of the thread, str0: its first streamed row,
+// columns TX apart.  The loop over the columns is rolled: with a mask test per pair written out, one masked tile cost more
+// in fetching its code (64 copies) than in computing: causal with a window, B1 H4 S50 D64, forward, cold: 86 us against 23
+// rolled.
+template <int TX, int NJ, bool OWN_KEYS>
+__device__ __forceinline__ uint64_t keep_bits(const AttnParams& p, int b, int own0, int str0, int q_lim, int k_len, bool masked) {
+  uint64_t bits = 0;
+#pragma unroll 1
+  for (int j = 0; j < NJ; ++j) {
+    const int str = str0 + TX * j;
+    const uint32_t live = OWN_KEYS ? (str < q_lim ? low_bits(k_len - own0) : 0u) : (str < k_len ? low_bits(q_lim - own0) : 0u);
+    uint32_t keep = live;
+    if (masked && live) {
+      const int q = (OWN_KEYS ? str : own0) + p.input_pos, kv = OWN_KEYS ? own0 : str;
+      keep = clause_bits<OWN_KEYS>(live, p.mask_flags, p.window, p.prefix_len, p.doc_q, p.doc_kv, p.doc_stride, b, q, kv);
+      for (int i = 0; i < p.n_or; ++i) {
+        const MaskClause& o = p.or_clause[i];
+        keep |= clause_bits<OWN_KEYS>(live, o.flags, o.window, o.prefix_len, o.doc_q, o.doc_kv, o.doc_stride, b, q, kv);
+      }
+    }
+    bits |= (uint64_t)keep << (RT * j);
+  }
+  return bits;
+}
+// The score mods of one (batch entry, query head): score_additive, score_apply and score_vjp with the table's base worked out
+// once and one tanh for a score and its derivative.
+struct ScoreMods {
+  float slope;
+  const float* bias;           // table of this batch entry and head, or null
+  size_t bias0;
+  __device__ __forceinline__ ScoreMods(const AttnParams& p, int b, int h)
+      : slope((p.score_flags & TYLO_SCORE_ALIBI) ? p.slopes[h] : 0.f), bias(nullptr), bias0(0) {
+    if (p.score_flags & TYLO_SCORE_BIAS) { bias0 = bias_index(p, b, h, 0, 0); bias = p.bias + bias0; }
+  }
+  // the additive mods of four pairs: keys kv.. of one row with KEYS, rows row.. at one key otherwise.  Pairs outside the problem
+  // take the nearest one inside (the table is not read beyond its end); their scores are not used.
+  template <bool KEYS>
+  __device__ __forceinline__ void additive(const AttnParams& p, int row, int kv, float (&add)[4]) const {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) add[i] = slope * (float)((KEYS ? row : row + i) + p.input_pos - (KEYS ? kv + i : kv));
+    if (bias) {          // one branch for the four, so that their loads are in flight together
+      float t[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) t[i] = bias[(size_t)min(KEYS ? row : row + i, p.Sq - 1) * p.Sk + min(KEYS ? kv + i : kv, p.Sk - 1)];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) add[i] += t[i];
+    }
+  }
+  // the modded score of the scaled score s0; d_add, d_s0: its derivatives by the additive mods and by s0
+  __device__ __forceinline__ float apply(const AttnParams& p, float s0, float add, float& d_add, float& d_s0) const {
+    d_add = 1.f; d_s0 = 1.f;
+    if (!(p.score_flags & TYLO_SCORE_SOFTCAP)) return s0 + add;
+    const bool cap_first = p.score_flags & TYLO_SCORE_SOFTCAP_FIRST;
+    const float th = tanhf((cap_first ? s0 : s0 + add) / p.cap), d = 1.f - th * th;
+    d_s0 = d;
+    if (!cap_first) d_add = d;
+    return cap_first ? p.cap * th + add : p.cap * th;
+  }
+};
 template <int TX, typename Op> __device__ __forceinline__ float row_reduce(float v, Op op) {
 #pragma unroll
   for (int o = TX / 2; o > 0; o >>= 1) v = op(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -200,7 +294,7 @@ fwd_kernel(float* __restrict__ O, const float* __restrict__ Q, const float* __re
   const float* Qg = Q + (size_t)(b * p.H + h) * p.Sq * p.Dk;
   const float* Kg = K + (size_t)(b * p.Hkv + hk) * p.Sk * p.Dk;
   const float* Vg = V + (size_t)(b * p.Hkv + hk) * p.Sk * p.Dk;
-  const float slope = (p.score_flags & TYLO_SCORE_ALIBI) ? p.slopes[h] : 0.f;
+  const ScoreMods mods(p, b, h);
   const bool modded = p.score_flags != 0;
   const float c = p.scale * kLog2e;
 
@@ -230,16 +324,23 @@ fwd_kernel(float* __restrict__ O, const float* __restrict__ Q, const float* __re
     cp_commit();
     float s[RT][NJ];
     dot_tile<D, NJ, true>(sQ, sK, ty, tx, s);
+    __syncwarp();              // a warp writes and reads only its own rows of P
     if (modded) {
-#pragma unroll
-      for (int i = 0; i < RT; ++i) {
-        const int row = min(q0 + RT * ty + i, p.Sq - 1);
-#pragma unroll
-        for (int j = 0; j < NJ; ++j) {
-          const int kv = min(kv0 + tx + TX * j, p.Sk - 1);
-          s[i][j] = score_apply(p, s[i][j] * p.scale, score_additive(p, slope, b, h, row, row + p.input_pos, kv)) * kLog2e;
-        }
+      // through the thread's own elements of P, four at a time in a rolled loop (see keep_bits); columns that no row can
+      // see are left as they are
+      put_transposed<D, NJ>(sP, ty, tx, s);
+      const int ne = 2 * min(NJ, (hi - kv0 + TX - 1) / TX);
+#pragma unroll 1
+      for (int e = 0; e < ne; ++e) {
+        const int j = e >> 1, i0 = 4 * (e & 1);
+        float4* u = reinterpret_cast<float4*>(sP + (tx + TX * j) * LDU + RT * ty + i0);
+        const float4 raw = *u;
+        float add[4], da, ds;
+        mods.additive<false>(p, q0 + RT * ty + i0, kv0 + tx + TX * j, add);
+        *u = make_float4(mods.apply(p, raw.x * p.scale, add[0], da, ds) * kLog2e, mods.apply(p, raw.y * p.scale, add[1], da, ds) * kLog2e,
+                         mods.apply(p, raw.z * p.scale, add[2], da, ds) * kLog2e, mods.apply(p, raw.w * p.scale, add[3], da, ds) * kLog2e);
       }
+      get_transposed<D, NJ>(sP, ty, tx, s);
     } else {
 #pragma unroll
       for (int i = 0; i < RT; ++i)
@@ -248,15 +349,11 @@ fwd_kernel(float* __restrict__ O, const float* __restrict__ Q, const float* __re
     }
     const bool masked = needs_mask(p, q0, kv0, BR);
     if (masked || kv0 + BR > k_len) {
+      const uint64_t bits = keep_bits<TX, NJ, false>(p, b, q0 + RT * ty, kv0 + tx, p.Sq, k_len, masked);
 #pragma unroll
-      for (int i = 0; i < RT; ++i) {
-        const int row = q0 + RT * ty + i;
+      for (int i = 0; i < RT; ++i)
 #pragma unroll
-        for (int j = 0; j < NJ; ++j) {
-          const int kv = kv0 + tx + TX * j;
-          if (!(row < p.Sq && kv < k_len && (!masked || mask_keep(p, b, row + p.input_pos, kv)))) s[i][j] = -INFINITY;
-        }
-      }
+        for (int j = 0; j < NJ; ++j) s[i][j] = (bits >> (RT * j + i)) & 1u ? s[i][j] : -INFINITY;
     }
 #pragma unroll
     for (int i = 0; i < RT; ++i) {
@@ -276,7 +373,6 @@ fwd_kernel(float* __restrict__ O, const float* __restrict__ Q, const float* __re
 #pragma unroll
       for (int e = 0; e < OC / 2; ++e) o[i][e] = sm100::mul_f32x2(o[i][e], sm100::pack_f32x2(alpha, alpha));
     }
-    __syncwarp();              // a warp writes and reads only its own rows of P
     put_transposed<D, NJ>(sP, ty, tx, s);
     cp_wait<0>();
     sh.sync();                 // V is there; everyone is done with K
@@ -445,15 +541,10 @@ __device__ __forceinline__ void bwd_tiles(float* sm, float* __restrict__ dA, flo
     const int q0 = OWN_KEYS ? str0 : own0, kv0 = OWN_KEYS ? own0 : str0;
     const bool masked = needs_mask(p, q0, kv0, OWN_KEYS ? BR : SB);
     const bool partial = masked || kv0 + (OWN_KEYS ? BR : SB) > k_len || q0 + (OWN_KEYS ? SB : BR) > q_lim;
-    const float slope = (p.score_flags & TYLO_SCORE_ALIBI) ? p.slopes[h] : 0.f;
-    // (query row, key) of element (i, j), and whether the pair takes part
-    auto row_of = [&](int i, int j) { return OWN_KEYS ? str0 + tx + TX * j : own0 + RT * ty + i; };
-    auto key_of = [&](int i, int j) { return OWN_KEYS ? own0 + RT * ty + i : str0 + tx + TX * j; };
+    const ScoreMods mods(p, b, h);
     auto lse_of = [&](int i, int j) { return OWN_KEYS ? sStat[tx + TX * j] : sOwn[RT * ty + i]; };
     auto delta_of = [&](int i, int j) { return OWN_KEYS ? sStat[SB + tx + TX * j] : sOwn[BR + RT * ty + i]; };
-    auto keep = [&](int row, int kv) {
-      return !partial || (row < q_lim && kv < k_len && (!masked || mask_keep(p, b, row + p.input_pos, kv)));
-    };
+    const uint64_t bits = partial ? keep_bits<TX, NJ, OWN_KEYS>(p, b, own0 + RT * ty, str0 + tx, q_lim, k_len, masked) : ~0ull;
     float s[RT][NJ];
     dot_tile<D, NJ, !OWN_KEYS>(sX1, sY1, ty, tx, s);
     if (!modded) {
@@ -461,7 +552,13 @@ __device__ __forceinline__ void bwd_tiles(float* sm, float* __restrict__ dA, flo
 #pragma unroll
       for (int i = 0; i < RT; ++i)
 #pragma unroll
-        for (int j = 0; j < NJ; ++j) s[i][j] = keep(row_of(i, j), key_of(i, j)) ? exp2f(fmaf(s[i][j], c, -lse_of(i, j))) : 0.f;
+        for (int j = 0; j < NJ; ++j) s[i][j] = exp2f(fmaf(s[i][j], c, -lse_of(i, j)));
+      if (partial) {
+#pragma unroll
+        for (int i = 0; i < RT; ++i)
+#pragma unroll
+          for (int j = 0; j < NJ; ++j) s[i][j] = (bits >> (RT * j + i)) & 1u ? s[i][j] : 0.f;
+      }
       put_transposed<D, NJ>(sU, ty, tx, s);
       __syncwarp();             // a warp writes and reads only its own rows of P and dS
       if constexpr (OWN_KEYS) acc_tile<D, SB>(sU, sY2, ty, tx, acc1);
@@ -482,44 +579,62 @@ __device__ __forceinline__ void bwd_tiles(float* sm, float* __restrict__ dA, flo
         }
       }
     } else {
-      // score mods: the raw products wait in shared memory; P, then dS with the mods' derivative at them
+      // score mods: the raw products wait in shared memory; P, then dS with the mods' derivative at them.  Four elements
+      // at a time in rolled loops (see keep_bits)
       put_transposed<D, NJ>(sU, ty, tx, s);
-      __syncwarp();
-      auto element = [&](float raw, int i, int j, float dp, float& at_add, float& ds) {       // returns p
-        const int row = row_of(i, j), kv = key_of(i, j);
-        at_add = 0.f; ds = 0.f;
-        if (!keep(row, kv)) return 0.f;
-        const float s0 = raw * p.scale, add = score_additive(p, slope, b, h, row, row + p.input_pos, kv);
-        const float pr = exp2f(score_apply(p, s0, add) * kLog2e - lse_of(i, j));
-        ds = score_vjp(p, s0, add, pr * (dp - delta_of(i, j)), &at_add) * p.scale;
+      auto row_of = [&](int i, int j) { return OWN_KEYS ? str0 + tx + TX * j : own0 + RT * ty + i; };
+      auto key_of = [&](int i, int j) { return OWN_KEYS ? own0 + RT * ty + i : str0 + tx + TX * j; };
+      auto element = [&](float raw, float add, int i, int j, float dp, float& ds) {       // returns p
+        ds = 0.f;
+        if (!((bits >> (RT * j + i)) & 1u)) return 0.f;
+        float d_add, d_s0;
+        const float pr = exp2f(mods.apply(p, raw * p.scale, add, d_add, d_s0) * kLog2e - lse_of(i, j));
+        const float g = pr * (dp - delta_of(i, j)), at_add = g * d_add;
+        ds = g * d_s0 * p.scale;
+        if (!OWN_KEYS) {      // parameter gradients: the dQ side meets every pair once (mods.jl:296-313)
+          const int row = row_of(i, j), kv = key_of(i, j);
+          slope_acc += at_add * (float)(row + p.input_pos - kv);
+          if (mods.bias && p.d_bias) atomicAdd(p.d_bias + mods.bias0 + (size_t)row * p.Sk + kv, at_add);
+        }
         return pr;
       };
-      float at_add, ds;
       if constexpr (OWN_KEYS) {
-        // (P of this thread's elements goes to its place, the raw products into registers, and back)
-#pragma unroll
-        for (int i = 0; i < RT; ++i)
-#pragma unroll
-          for (int j = 0; j < NJ; ++j) sU[(tx + TX * j) * LDU + RT * ty + i] = element(s[i][j], i, j, 0.f, at_add, ds);
+        float ds;
+        // (P of this thread's elements goes to its place, and the raw products back)
+#pragma unroll 1
+        for (int e = 0; e < 2 * NJ; ++e) {
+          const int j = e >> 1, i0 = 4 * (e & 1);
+          float4* u = reinterpret_cast<float4*>(sU + (tx + TX * j) * LDU + RT * ty + i0);
+          float4 w = *u;
+          float add[4];
+          mods.additive<OWN_KEYS>(p, row_of(i0, j), key_of(i0, j), add);
+          w.x = element(w.x, add[0], i0, j, 0.f, ds); w.y = element(w.y, add[1], i0 + 1, j, 0.f, ds);
+          w.z = element(w.z, add[2], i0 + 2, j, 0.f, ds); w.w = element(w.w, add[3], i0 + 3, j, 0.f, ds);
+          *u = w;
+        }
         __syncwarp();
         acc_tile<D, SB>(sU, sY2, ty, tx, acc1);
         __syncwarp();
         put_transposed<D, NJ>(sU, ty, tx, s);
       }
       dot_tile<D, NJ, !OWN_KEYS>(sX2, sY2, ty, tx, s);
+#pragma unroll 1
+      for (int e = 0; e < 2 * NJ; ++e) {
+        const int j = e >> 1, i0 = 4 * (e & 1);
+        float4* u = reinterpret_cast<float4*>(sU + (tx + TX * j) * LDU + RT * ty + i0);
+        const float4 raw = *u;
+        float4 w;
+        float add[4];
+        mods.additive<OWN_KEYS>(p, row_of(i0, j), key_of(i0, j), add);
+        element(raw.x, add[0], i0, j, s[0][0], w.x); element(raw.y, add[1], i0 + 1, j, s[1][0], w.y);
+        element(raw.z, add[2], i0 + 2, j, s[2][0], w.z); element(raw.w, add[3], i0 + 3, j, s[3][0], w.w);
+        *u = w;
+        // the next four dP move up to the front (registers cannot be indexed)
 #pragma unroll
-      for (int i = 0; i < RT; ++i)
+        for (int k = 0; k < NJ; ++k)
 #pragma unroll
-        for (int j = 0; j < NJ; ++j) {
-          float* u = sU + (tx + TX * j) * LDU + RT * ty + i;
-          element(*u, i, j, s[i][j], at_add, ds);
-          if (!OWN_KEYS) {      // parameter gradients: the dQ side meets every pair once (mods.jl:296-313)
-            const int row = row_of(i, j), kv = key_of(i, j);
-            slope_acc += at_add * (float)(row + p.input_pos - kv);
-            if (p.d_bias && (p.score_flags & TYLO_SCORE_BIAS) && keep(row, kv)) atomicAdd(p.d_bias + bias_index(p, b, h, row, kv), at_add);
-          }
-          *u = ds;
-        }
+          for (int i = 0; i < 4; ++i) { s[i][k] = s[i + 4][k]; if (k + 1 < NJ) s[i + 4][k] = s[i][k + 1]; }
+      }
     }
     __syncwarp();
     acc_tile<D, SB>(sU, sY1, ty, tx, acc2);
@@ -601,8 +716,28 @@ static int32_t launch_bwd(float* dQ, float* dK, float* dV, const float* Q, const
 }  // namespace f32
 
 // (the entry points refuse arrays that are not 16-byte aligned)
-bool attn_f32_supported(const AttnParams& p, int32_t dtype) {
+static bool f32_covers(const AttnParams& p, int32_t dtype) {
   return dtype == TYLO_F32 && p.Dk == p.Dv && p.Dk % 4 == 0 && p.Dk >= 4 && p.Dk <= 128 && !p.bm_count;
+}
+
+// Where the 32 x 32 tiles of attn_generic.cu are still the better ones: calls of one key tile, in which one group of threads
+// works while the others (three of four at head dims up to 64) wait, on one CTA per SM where the general kernel has four or
+// more.  Times in us, general kernel / this one, B 64 H 8 unless stated:
+bool attn_fwd_f32_preferred(const AttnParams& p, int32_t dtype) {
+  if (!f32_covers(p, dtype)) return false;
+  const bool cap = p.score_flags & TYLO_SCORE_SOFTCAP;
+  const bool waves = (long long)((p.Sq + f32::BR - 1) / f32::BR) * p.H * p.B > sm_count();      // more CTAs than SMs
+  if (p.Dk > 64)               // two groups: S 32 D 128 55 / 57, with a soft cap 57 / 71; from 33 on ours: 109 / 62
+    return !(waves && p.Sq <= 32 && p.Sk <= 32);
+  if (p.Sk <= 32) return false;                                      // S 32 D 64: 37 / 60; 1 x 32: 33 / 65; B 1 H 4 1 x 32 warm: 7.4 / 10
+  if (cap && p.Sk <= 64) return false;                               // (64 tanh in a row per thread) S 50 D 64: 84 / 117
+  if (waves && p.Sq <= 32) return !(p.Sk <= 64 || (cap && p.Sk <= 256));    // bias 8 x 64 D 64: 35 / 50; soft cap 32 x 100: 58 / 72
+  return true;
+}
+bool attn_bwd_f32_preferred(const AttnParams& p, int32_t dtype) {
+  if (!f32_covers(p, dtype)) return false;
+  // score mods on a single half-empty tile, CTAs for more than three waves: bias S 32 D 64 152 / 180 (B 20: 82 / 73, B 1: 53 / 29)
+  return !(p.Dk <= 64 && p.score_flags && p.Sq <= 32 && p.Sk <= 32 && (long long)(p.H + p.Hkv) * p.B > 3 * sm_count());
 }
 
 int32_t attn_fwd_f32(void* O, const void* Q, const void* K, const void* V, float* M, float* L, const AttnParams& p, cudaStream_t st) {
