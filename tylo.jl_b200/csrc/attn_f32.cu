@@ -10,10 +10,10 @@
 // the streamed tiles in turn, each with its own tiles, statistics and accumulators, and are merged once at the end: small
 // problems have about one CTA per SM, and one group's loads and exponentials run under the other groups' FMAs.
 //
-// Packed pairs (fma.rn.f32x2) are used where their accumulators fit: they take half the issue slots, and with more warps
-// than the registers allow here twice the rate.  Measured, forward + backward: B2 H8 S512 D64 825 us on the 2 x 2 patches,
-// 209 with 4 x 8 patches, 204 with 8 x 8, 197 with packed pairs, 201 with short chains; the FMA pipes are 46 % / 40 % busy (forward / backward), eight
-// warps per SM do not hide the shared-memory latency.
+// Packed pairs (fma.rn.f32x2) are used where their accumulators fit: they take half the issue slots, and with 32 warps per SM
+// twice the rate (242 FMA per clock; with the eight warps that the registers allow here 125, as many as fmaf).  Every sum is
+// kept in short chains (see dot_tile and acc_tile).  Forward + backward of B2 H8 S512 D64: 825 us on the 2 x 2 patches of
+// attn_generic.cu, 174 here; eight warps per SM do not hide the shared-memory latency.
 //
 // Forward: online softmax per group.  Backward: no atomics on dQ / dK / dV; dK / dV CTAs (own 64 keys, sum the query heads
 // of the group) and dQ CTAs (own 64 queries) share one launch, heaviest first, so that both fill the SMs together.
@@ -26,6 +26,10 @@ namespace f32 {
 constexpr int BR = 64, RT = 8;     // rows a CTA owns, rows of a thread
 constexpr int kThreads = 256;
 constexpr int LDU = BR + 4;        // probabilities / score gradients: [streamed row][own row]
+// Up to so many keys, and at head dim 128, dot_tile takes its finer form (template argument FINE): the fewer keys, the more the
+// rounding of the scores outweighs that of the sums over the keys, and at 128 it costs nothing.  Relative error of O against 64
+// bits, D 64: 144 keys 1.96e-7 (2.09e-7 otherwise, 2.06e-7 in attn_generic.cu), 512 keys 2.20e-7 without it (2.28e-7 there).
+constexpr int kFineKeys = 384;
 
 // TX threads side by side over a tile's columns, 8 of them down its rows: a group of 64 or 128 threads.
 template <int D> struct Shape {
@@ -54,8 +58,12 @@ __device__ __forceinline__ void load_tile(float* dst, const float* __restrict__ 
 }
 
 // out[i][j] = X[8 ty + i] . Y[tx + TX j].  PAIR: even and odd columns of the head dim in the two halves of packed pairs
-// (fma.rn.f32x2 has twice the rate of fmaf), for twice the accumulators.
-template <int D, int NJ, bool PAIR>
+// (fma.rn.f32x2: half the instructions), for twice the accumulators.  FINE: the products of four columns are summed on their own
+// before they join the accumulator, so that it rounds D / 4 times and not D / 2 times per half: an instruction more per four
+// columns and pair (512 x 512, D 64: 43 -> 49 us forward; at D 128, where the loads hide it, 74 either way).  The fine form is
+// paired in every kernel, spilling or not: scores that round alike in the forward and in both halves of the backward make P of a
+// row with few keys exact (dV of 49 causal rows, D 64: error 1.13 times that of attn_generic.cu otherwise, 0.94 so).
+template <int D, int NJ, bool PAIR, bool FINE>
 __device__ __forceinline__ void dot_tile(const float* __restrict__ X, const float* __restrict__ Y, int ty, int tx, float (&out)[RT][NJ]) {
   constexpr int TX = Shape<D>::TX;
   const float* x = X + RT * ty * (D + 4);
@@ -75,7 +83,9 @@ __device__ __forceinline__ void dot_tile(const float* __restrict__ X, const floa
       for (int j = 0; j < NJ; ++j) {
         const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(y + j * TX * (D + 4) + c);
 #pragma unroll
-        for (int i = 0; i < RT; ++i) acc[i][j] = sm100::fma_f32x2(a[i].y, b.y, sm100::fma_f32x2(a[i].x, b.x, acc[i][j]));
+        for (int i = 0; i < RT; ++i)
+          acc[i][j] = FINE ? sm100::add_f32x2(acc[i][j], sm100::fma_f32x2(a[i].y, b.y, sm100::mul_f32x2(a[i].x, b.x)))
+                           : sm100::fma_f32x2(a[i].y, b.y, sm100::fma_f32x2(a[i].x, b.x, acc[i][j]));
       }
     }
 #pragma unroll
@@ -103,27 +113,51 @@ __device__ __forceinline__ void dot_tile(const float* __restrict__ X, const floa
   }
 }
 
-// acc[i], columns 4 j + e (in pairs) += sum_n U[n][8 ty + i] Y[n][4 TX j + 4 tx + e]
-template <int D, int ROWS>
-__device__ __forceinline__ void acc_tile(const float* __restrict__ U, const float* __restrict__ Y, int ty, int tx, uint64_t (&acc)[RT][Shape<D>::OC / 2]) {
-  constexpr int TX = Shape<D>::TX, OC = Shape<D>::OC;
+// acc[i], columns 4 j + e (in pairs) = acc[i] f[i] (f only with SCALE) + sum_n U[n][8 ty + i] Y[n][4 TX j + 4 tx + e].  The rows are
+// summed in PARTS sums of their own, in the registers of the scores, which are free by then: an accumulator that runs through
+// all rows rounds once per row (dK of 1,200 rows, D 128: error 6.4e-7 in one chain, 3.7e-7 so; of 512, D 64: 4.0e-7, 3.5e-7).
+template <int D, int ROWS, int PARTS, bool SCALE>
+__device__ __forceinline__ void acc_tile(const float* __restrict__ U, const float* __restrict__ Y, int ty, int tx,
+                                         uint64_t (&acc)[RT][Shape<D>::OC / 2], const float (&f)[RT]) {
+  constexpr int TX = Shape<D>::TX, OC = Shape<D>::OC, N = ROWS / PARTS;
+  static_assert(ROWS % PARTS == 0, "whole parts");
   const float* u = U + RT * ty;
   const float* y = Y + 4 * tx;
+#pragma unroll 1
+  for (int part = 0; part < PARTS; ++part) {
+    uint64_t t[RT][OC / 2];
+#pragma unroll
+    for (int i = 0; i < RT; ++i)
+#pragma unroll
+      for (int e = 0; e < OC / 2; ++e) t[i][e] = 0ull;
 #pragma unroll 4
-  for (int n = 0; n < ROWS; ++n) {
-    const float4 p0 = *reinterpret_cast<const float4*>(u + n * LDU), p1 = *reinterpret_cast<const float4*>(u + n * LDU + 4);
-    const float pi[RT] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
+    for (int n = part * N; n < (part + 1) * N; ++n) {
+      const float4 p0 = *reinterpret_cast<const float4*>(u + n * LDU), p1 = *reinterpret_cast<const float4*>(u + n * LDU + 4);
+      const float pi[RT] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
 #pragma unroll
-    for (int j = 0; j < OC / 4; ++j) {
-      const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(y + n * (D + 4) + 4 * TX * j);
+      for (int j = 0; j < OC / 4; ++j) {
+        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(y + n * (D + 4) + 4 * TX * j);
 #pragma unroll
-      for (int i = 0; i < RT; ++i) {
-        const uint64_t p2 = sm100::pack_f32x2(pi[i], pi[i]);
-        acc[i][2 * j] = sm100::fma_f32x2(p2, v.x, acc[i][2 * j]);
-        acc[i][2 * j + 1] = sm100::fma_f32x2(p2, v.y, acc[i][2 * j + 1]);
+        for (int i = 0; i < RT; ++i) {
+          const uint64_t p2 = sm100::pack_f32x2(pi[i], pi[i]);
+          t[i][2 * j] = sm100::fma_f32x2(p2, v.x, t[i][2 * j]);
+          t[i][2 * j + 1] = sm100::fma_f32x2(p2, v.y, t[i][2 * j + 1]);
+        }
       }
     }
+#pragma unroll
+    for (int i = 0; i < RT; ++i) {
+      const float fi = part == 0 ? f[i] : 1.f;
+      const uint64_t f2 = sm100::pack_f32x2(fi, fi);
+#pragma unroll
+      for (int e = 0; e < OC / 2; ++e) acc[i][e] = SCALE ? sm100::fma_f32x2(acc[i][e], f2, t[i][e]) : sm100::add_f32x2(acc[i][e], t[i][e]);
+    }
   }
+}
+template <int D, int ROWS, int PARTS>
+__device__ __forceinline__ void acc_tile(const float* __restrict__ U, const float* __restrict__ Y, int ty, int tx, uint64_t (&acc)[RT][Shape<D>::OC / 2]) {
+  const float none[RT] = {};
+  acc_tile<D, ROWS, PARTS, false>(U, Y, ty, tx, acc, none);
 }
 // U[tx + TX j][8 ty + i] = v[i][j]
 template <int D, int NJ>
@@ -267,10 +301,11 @@ template <int TX, typename Op> __device__ __forceinline__ float row_reduce(float
 template <int D> struct FwdSmem {
   static constexpr int kTile = BR * (D + 4), kU = BR * LDU;           // floats
   static constexpr int kGroup = 2 * kTile + kU;                        // K, V, P of one group
-  static constexpr int kBytes = (kTile + Shape<D>::kGroups * kGroup) * 4;      // 128 KB, 221 KB, 199 KB for D = 32, 64, 128
+  static constexpr int kBytes = (kTile + Shape<D>::kGroups * kGroup) * 4;      // 149 KB, 221 KB, 199 KB for D = 32, 64, 128
+  static constexpr int kParts = 4;                                     // sums of 16 keys
 };
 
-template <int D>
+template <int D, bool FINE>
 __global__ void __launch_bounds__(kThreads, 1)
 fwd_kernel(float* __restrict__ O, const float* __restrict__ Q, const float* __restrict__ K, const float* __restrict__ V,
            float* __restrict__ Mout, float* __restrict__ Lout, const AttnParams p) {
@@ -298,6 +333,7 @@ fwd_kernel(float* __restrict__ O, const float* __restrict__ Q, const float* __re
   const bool modded = p.score_flags != 0;
   const float c = p.scale * kLog2e;
 
+
   int lo, hi;
   kv_range(p, q0 + p.input_pos, min(q0 + BR, p.Sq) - 1 + p.input_pos, k_len, &lo, &hi);
   const int t0 = lo / BR, t1 = hi > lo ? (hi - 1) / BR + 1 : t0;
@@ -323,7 +359,7 @@ fwd_kernel(float* __restrict__ O, const float* __restrict__ Q, const float* __re
     load_tile<D, BR, GT>(sV, Vg, kv0, k_len, p.Dk, tid);
     cp_commit();
     float s[RT][NJ];
-    dot_tile<D, NJ, true>(sQ, sK, ty, tx, s);
+    dot_tile<D, NJ, true, FINE>(sQ, sK, ty, tx, s);
     __syncwarp();              // a warp writes and reads only its own rows of P
     if (modded) {
       // through the thread's own elements of P, four at a time in a rolled loop (see keep_bits); columns that no row can
@@ -355,6 +391,7 @@ fwd_kernel(float* __restrict__ O, const float* __restrict__ Q, const float* __re
 #pragma unroll
         for (int j = 0; j < NJ; ++j) s[i][j] = (bits >> (RT * j + i)) & 1u ? s[i][j] : -INFINITY;
     }
+    float f[RT];
 #pragma unroll
     for (int i = 0; i < RT; ++i) {
       float mx = s[i][0];
@@ -370,15 +407,14 @@ fwd_kernel(float* __restrict__ O, const float* __restrict__ Q, const float* __re
       }
       l[i] = l[i] * alpha + ps;
       m[i] = mn;
-#pragma unroll
-      for (int e = 0; e < OC / 2; ++e) o[i][e] = sm100::mul_f32x2(o[i][e], sm100::pack_f32x2(alpha, alpha));
+      f[i] = alpha;
     }
     put_transposed<D, NJ>(sP, ty, tx, s);
     cp_wait<0>();
     sh.sync();                 // V is there; everyone is done with K
     if (t + NG < t1) load_tile<D, BR, GT>(sK, Kg, (t + NG) * BR, k_len, p.Dk, tid);
     cp_commit();
-    acc_tile<D, BR>(sP, sV, ty, tx, o);
+    acc_tile<D, BR, SM::kParts, true>(sP, sV, ty, tx, o, f);
   }
 
   // merge of the groups: each leaves its rows in its own K tile and its statistics in its own P; every thread then takes an
@@ -425,6 +461,7 @@ template <int D> struct BwdSmem {
   static constexpr int SB = D <= 32 ? 64 : 48;
   static constexpr int kOwn = BR * (D + 4), kTile = SB * (D + 4), kU = SB * LDU;
   static constexpr int kGroup = 2 * kTile + kU + 2 * SB;               // Y1, Y2, P / dS, statistics
+  static constexpr int kParts = D == 128 ? 1 : 2;                      // sums of 48 rows, 24 (64), 32 (32)
   static constexpr int kBytes = (2 * kOwn + 2 * BR + Shape<D>::kGroups * kGroup) * 4;
   static_assert(kGroup >= kOwn, "a group's sum is left in its own tiles");
 };
@@ -446,7 +483,7 @@ delta_kernel(float* __restrict__ Delta, const float* __restrict__ O, const float
 
 // OWN_KEYS: own 64 keys of a KV head, stream the queries of its group (dV += P^T dO, dK += dS^T Q); otherwise own 64 queries,
 // stream keys (dQ += dS K).  Own rows are the rows of T1 = X1 Y1^T (scores) and T2 = X2 Y2^T (dP).
-template <int D, bool OWN_KEYS>
+template <int D, bool OWN_KEYS, bool FINE>
 __device__ __forceinline__ void bwd_tiles(float* sm, float* __restrict__ dA, float* __restrict__ dB, const float* __restrict__ Q,
                                           const float* __restrict__ K, const float* __restrict__ V, const float* __restrict__ dO,
                                           const float* __restrict__ Mst, const float* __restrict__ Lst,
@@ -546,7 +583,7 @@ __device__ __forceinline__ void bwd_tiles(float* sm, float* __restrict__ dA, flo
     auto delta_of = [&](int i, int j) { return OWN_KEYS ? sStat[SB + tx + TX * j] : sOwn[BR + RT * ty + i]; };
     const uint64_t bits = partial ? keep_bits<TX, NJ, OWN_KEYS>(p, b, own0 + RT * ty, str0 + tx, q_lim, k_len, masked) : ~0ull;
     float s[RT][NJ];
-    dot_tile<D, NJ, !OWN_KEYS>(sX1, sY1, ty, tx, s);
+    dot_tile<D, NJ, !OWN_KEYS || FINE, FINE>(sX1, sY1, ty, tx, s);
     if (!modded) {
       // P into shared memory, dV from it; dS takes its place element by element (each thread its own)
 #pragma unroll
@@ -561,8 +598,8 @@ __device__ __forceinline__ void bwd_tiles(float* sm, float* __restrict__ dA, flo
       }
       put_transposed<D, NJ>(sU, ty, tx, s);
       __syncwarp();             // a warp writes and reads only its own rows of P and dS
-      if constexpr (OWN_KEYS) acc_tile<D, SB>(sU, sY2, ty, tx, acc1);
-      dot_tile<D, NJ, !OWN_KEYS>(sX2, sY2, ty, tx, s);
+      if constexpr (OWN_KEYS) acc_tile<D, SB, SM::kParts>(sU, sY2, ty, tx, acc1);
+      dot_tile<D, NJ, !OWN_KEYS || FINE, FINE>(sX2, sY2, ty, tx, s);
       __syncwarp();
 #pragma unroll
       for (int j = 0; j < NJ; ++j) {
@@ -613,11 +650,11 @@ __device__ __forceinline__ void bwd_tiles(float* sm, float* __restrict__ dA, flo
           *u = w;
         }
         __syncwarp();
-        acc_tile<D, SB>(sU, sY2, ty, tx, acc1);
+        acc_tile<D, SB, SM::kParts>(sU, sY2, ty, tx, acc1);
         __syncwarp();
         put_transposed<D, NJ>(sU, ty, tx, s);
       }
-      dot_tile<D, NJ, !OWN_KEYS>(sX2, sY2, ty, tx, s);
+      dot_tile<D, NJ, !OWN_KEYS || FINE, FINE>(sX2, sY2, ty, tx, s);
 #pragma unroll 1
       for (int e = 0; e < 2 * NJ; ++e) {
         const int j = e >> 1, i0 = 4 * (e & 1);
@@ -637,7 +674,7 @@ __device__ __forceinline__ void bwd_tiles(float* sm, float* __restrict__ dA, flo
       }
     }
     __syncwarp();
-    acc_tile<D, SB>(sU, sY1, ty, tx, acc2);
+    acc_tile<D, SB, SM::kParts>(sU, sY1, ty, tx, acc2);
   }
 
   // sums over the groups, one output at a time, through each group's own tiles
@@ -673,7 +710,7 @@ __device__ __forceinline__ void bwd_tiles(float* sm, float* __restrict__ dA, flo
   }
 }
 
-template <int D>
+template <int D, bool FINE>
 __global__ void __launch_bounds__(kThreads, 1)
 bwd_kernel(float* __restrict__ dQ, float* __restrict__ dK, float* __restrict__ dV, const float* __restrict__ Q,
            const float* __restrict__ K, const float* __restrict__ V, const float* __restrict__ dO, const float* __restrict__ Mst,
@@ -683,20 +720,21 @@ bwd_kernel(float* __restrict__ dQ, float* __restrict__ dK, float* __restrict__ d
   // key blocks and the last query blocks see the most
   if ((int)blockIdx.x < n_keys) {
     const int heads = p.Hkv * p.B, hb = blockIdx.x % heads;
-    bwd_tiles<D, true>(sm, dK, dV, Q, K, V, dO, Mst, Lst, Delta, p, hb / p.Hkv, hb % p.Hkv, (int)(blockIdx.x / heads) * BR);
+    bwd_tiles<D, true, FINE>(sm, dK, dV, Q, K, V, dO, Mst, Lst, Delta, p, hb / p.Hkv, hb % p.Hkv, (int)(blockIdx.x / heads) * BR);
   } else {
     const int i = blockIdx.x - n_keys, heads = p.H * p.B, hb = i % heads, nqt = (p.Sq + BR - 1) / BR;
-    bwd_tiles<D, false>(sm, dQ, nullptr, Q, K, V, dO, Mst, Lst, Delta, p, hb / p.H, hb % p.H, (nqt - 1 - i / heads) * BR);
+    bwd_tiles<D, false, FINE>(sm, dQ, nullptr, Q, K, V, dO, Mst, Lst, Delta, p, hb / p.H, hb % p.H, (nqt - 1 - i / heads) * BR);
   }
 }
 
 template <int D>
 static int32_t launch_fwd(float* O, const float* Q, const float* K, const float* V, float* M, float* L, const AttnParams& p,
                           cudaStream_t st) {
-  TYLO_CUDA_OK(cudaFuncSetAttribute(fwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdSmem<D>::kBytes));
+  auto kern = D == 128 || p.Sk <= kFineKeys ? fwd_kernel<D, true> : fwd_kernel<D, D == 128>;
+  TYLO_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdSmem<D>::kBytes));
   const long long grid = (long long)((p.Sq + BR - 1) / BR) * p.H * p.B;
   TYLO_REQUIRE(grid <= 0x7fffffffLL, TYLO_ERR_UNSUPPORTED, "attention: problem too large for one launch");
-  fwd_kernel<D><<<(unsigned)grid, kThreads, FwdSmem<D>::kBytes, st>>>(O, Q, K, V, M, L, p);
+  kern<<<(unsigned)grid, kThreads, FwdSmem<D>::kBytes, st>>>(O, Q, K, V, M, L, p);
   return check_launch("attn_fwd_f32");
 }
 
@@ -708,8 +746,9 @@ static int32_t launch_bwd(float* dQ, float* dK, float* dV, const float* Q, const
   TYLO_REQUIRE(n_keys + n_q <= 0x7fffffffLL, TYLO_ERR_UNSUPPORTED, "attention backward: problem too large");
   delta_kernel<<<(unsigned)((rows + 31) / 32), 256, 0, st>>>(Delta, O, dO, rows, p.Dk);
   if (int32_t rc = check_launch("attn_bwd_f32_delta")) return rc;
-  TYLO_CUDA_OK(cudaFuncSetAttribute(bwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem<D>::kBytes));
-  bwd_kernel<D><<<(unsigned)(n_keys + n_q), kThreads, BwdSmem<D>::kBytes, st>>>(dQ, dK, dV, Q, K, V, dO, M, L, Delta, p, (int)n_keys);
+  auto kern = D == 128 || p.Sk <= kFineKeys ? bwd_kernel<D, true> : bwd_kernel<D, D == 128>;
+  TYLO_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem<D>::kBytes));
+  kern<<<(unsigned)(n_keys + n_q), kThreads, BwdSmem<D>::kBytes, st>>>(dQ, dK, dV, Q, K, V, dO, M, L, Delta, p, (int)n_keys);
   return check_launch("attn_bwd_f32");
 }
 
