@@ -560,15 +560,15 @@ __device__ __forceinline__ void bwd_tiles(float* sm, float* __restrict__ dA, flo
   cp_commit();
   cp_wait<0>();
   __syncthreads();
-  // dK / dV: one query head of the group at a time, summed into the outputs head by head, so that an accumulator's chain is no
-  // longer than a head's share of rows
-  for (int g = 0; g < (OWN_KEYS ? p.G : 1); ++g) {
-  const int h = h0 + g;
 #pragma unroll
   for (int i = 0; i < RT; ++i)
 #pragma unroll
     for (int e = 0; e < OC / 2; ++e) { acc1[i][e] = 0ull; acc2[i][e] = 0ull; }
-  for (int n = grp; n < nt; n += NG) {
+  // dK / dV: the tiles of all query heads of the group are dealt over the groups of threads (head by head, groups of threads
+  // idled whenever a head has fewer tiles than there are groups, and every head paid for a merge)
+  const int total = OWN_KEYS ? nt * p.G : nt;
+  for (int u = grp; u < total; u += NG) {
+    const int n = OWN_KEYS ? u % nt : u, h = OWN_KEYS ? h0 + u / nt : h0;
     const int str0 = (t0 + n) * SB;
     sh.sync();                  // everyone is done with the tile before
     load_y(n, h);
@@ -693,17 +693,11 @@ __device__ __forceinline__ void bwd_tiles(float* sm, float* __restrict__ dA, flo
         const float4 x = *reinterpret_cast<const float4*>(gs + k * SM::kGroup + r * (D + 4) + col);
         t.x += x.x; t.y += x.y; t.z += x.z; t.w += x.w;
       }
-      if (col < p.Dk) {
-        float4* o = reinterpret_cast<float4*>(out + (base + row) * p.Dk + col);
-        if (g > 0) { const float4 q = *o; t.x += q.x; t.y += q.y; t.z += q.z; t.w += q.w; }     // (this thread's own earlier store)
-        *o = t;
-      }
+      if (col < p.Dk) *reinterpret_cast<float4*>(out + (base + row) * p.Dk + col) = t;
     }
   };
   if constexpr (OWN_KEYS) merge(acc1, dB);
   merge(acc2, dA);
-  __syncthreads();              // the groups' tiles have been read
-  }
   if (!OWN_KEYS && p.d_slopes && (p.score_flags & TYLO_SCORE_ALIBI)) {
     slope_acc = warp_reduce(slope_acc, SumOp());
     if (sh.lane == 0 && slope_acc != 0.f) atomicAdd(p.d_slopes + h0, slope_acc);
