@@ -87,3 +87,28 @@ def test_norm_rows(tylo, oracle, M, N, groups, dt):
     check(dX, dXr, dt, "ln dX")
     check(dW, dWr, dt, "ln dW", scale_hint=4 * float(np.abs(dWr).max()))
     check(dB, dBr, dt, "ln dB", scale_hint=4 * float(np.abs(dBr).max()))
+
+
+def test_norm_backward_of_the_most_rows(tylo):
+    """2^31 - 1 rows, the most that are accepted: the rows asked for ahead of the last ones lie beyond what an int holds."""
+    M, N, tail = 8, 2 ** 31 - 1, 20000
+    torch.cuda.empty_cache()
+    if torch.cuda.mem_get_info()[0] < 125e9:
+        pytest.skip("needs 115 GB")
+    X, dY, dX = (torch.ones(N, M, device="cuda", dtype=torch.bfloat16) for _ in range(3))
+    g = torch.Generator("cuda").manual_seed(1)
+    for t in (X, dY):
+        t[-tail:] = torch.randn(tail, M, generator=g, device="cuda").bfloat16()
+    W, dW = torch.ones(M, device="cuda", dtype=torch.bfloat16), torch.empty(M, device="cuda", dtype=torch.bfloat16)
+    cp = tylo.allocate_checkpoints_rms_norm(X, W)
+    tylo.rms_norm_(dX, X, W, eps=1e-6, checkpoints=cp)
+    d = tylo.Duplicated
+    tylo.grad_rms_norm_(d(dX, dY), d(X, dX), d(W, dW), checkpoints=cp, scratch=tylo.allocate_scratchspace_grad_rms_norm(X, W))
+    x = X[-tail:].double().requires_grad_()
+    y = x * torch.rsqrt((x * x).mean(-1, keepdim=True) + 1e-6)
+    y.backward(dY[-tail:].double())
+    err = (dX[-tail:].double() - x.grad).abs()
+    assert bool((err <= 2.0 ** -8 * x.grad.abs() + 1e-4).all())        # an ulp of bf16
+    assert bool((dX[:tail].float().abs() < 1e-5).all())               # rows of ones: dY is parallel to X
+    del X, dY, dX, cp
+    torch.cuda.empty_cache()

@@ -372,12 +372,13 @@ norm_bwd_kernel(T* __restrict__ dX, float* __restrict__ dWp, float* __restrict__
     g[j] = live ? (LAYER ? g[j] : g[j] + offset) : 0.f;
     dw[j] = 0.f; db[j] = 0.f;
   }
-  const int stride = (int)gridDim.x * R;        // (at most 296 x 15, see the launch)
+  // rows are counted in unsigned: N may be 2^31 - 1, and the row asked for ahead lies up to 2 x 296 x 15 beyond (see the launch)
+  const unsigned stride = gridDim.x * (unsigned)R, rows = (unsigned)N;
   Pack<T> x0, d0, x1, d1, x2, d2;
   x0.raw = d0.raw = x1.raw = d1.raw = x2.raw = d2.raw = make_uint4(0, 0, 0, 0);
   float r0 = 0.f, r1 = 0.f, r2 = 0.f, m0 = 0.f, m1 = 0.f, m2 = 0.f;
-  auto fetch = [&](int r, Pack<T>& x, Pack<T>& d, float& rs, float& mn) {
-    if ((unsigned)r < (unsigned)N) {
+  auto fetch = [&](unsigned r, Pack<T>& x, Pack<T>& d, float& rs, float& mn) {
+    if (r < rows) {
       if (live) { x.raw = ld_stream(X + (size_t)r * M + col); d.raw = ld_stream(dY + (size_t)r * M + col); }
       rs = Rstd[r];
       mn = LAYER ? Mean[r] : 0.f;
@@ -385,10 +386,10 @@ norm_bwd_kernel(T* __restrict__ dX, float* __restrict__ dWp, float* __restrict__
   };
   // rows in flight behind the current one: two for RMSNorm, one for LayerNorm (its extra accumulators
   // and statistics would otherwise push the 1024-thread CTA past 64 registers per thread)
-  int row = (int)blockIdx.x * R + rg;
+  unsigned row = blockIdx.x * (unsigned)R + rg;
   fetch(row, x0, d0, r0, m0);
   if constexpr (!LAYER) fetch(row + stride, x1, d1, r1, m1);
-  for (int par = 0; (unsigned)row < (unsigned)N; row += stride, par ^= 1) {
+  for (int par = 0; row < rows; row += stride, par ^= 1) {
     if constexpr (LAYER) fetch(row + stride, x1, d1, r1, m1);
     else fetch(row + 2 * stride, x2, d2, r2, m2);
     float s1 = 0.f, s2 = 0.f;
