@@ -85,3 +85,32 @@ def test_error_against_64_bits(tylo):
     for a, b, bound, name in zip(got, (ref.detach(), q.grad, k.grad, v.grad), (3.6e-7, 5.1e-7, 5.3e-7, 5.0e-7), ("O", "dQ", "dK", "dV")):
         err = float((a.double() - b).norm() / b.norm())
         assert err <= bound, f"{name}: {err:.2e} > {bound:.1e}"
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("D", [32, 64, 128])
+def test_ragged_backward(tylo, oracle, D, causal):
+    """Lengths of none, one, a tile less one, a tile and one, and all rows: each batch entry against the oracle on its own keys and
+    query blocks; keys beyond a length and query blocks beyond one get gradients of exactly zero."""
+    lens = [0, 1, 63, 65, 200]
+    B, H, Hkv, S = len(lens), 4, 2, 200
+    rng = np.random.default_rng(D)
+    Q, Q64 = draw(rng, (B, H, S, D), "f32"); K, K64 = draw(rng, (B, Hkv, S, D), "f32"); V, V64 = draw(rng, (B, Hkv, S, D), "f32")
+    dO, dO64 = draw(rng, (B, H, S, D), "f32")
+    n = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    kw = dict(causal=causal, k_lengths=n, q_lengths=n)
+    cp = tylo.allocate_checkpoints_attention(Q, K, V)
+    O = torch.zeros_like(Q)
+    tylo.attention_(O, Q, K, V, checkpoints=cp, **kw)
+    dQ, dK, dV = tylo.grad_attention(dO, Q, K, V, O, checkpoints=cp, **kw)
+    for b, k in enumerate(lens):
+        q = min(S, -(-k // 64) * 64)                  # query blocks of 64 rows that start below the length
+        assert not dQ[b, :, q:].any() and not dK[b, :, k:].any() and not dV[b, :, k:].any() and not O[b, :, q:].any()
+        if k == 0:
+            continue
+        okw = dict(mask=oracle.MaskSpec(causal=True) if causal else None)
+        args = (Q64[b:b + 1, :, :q], K64[b:b + 1, :, :k], V64[b:b + 1, :, :k])
+        check(O[b:b + 1, :, :q], oracle.flex_ref(*args, **okw), "f32", f"O of length {k}")
+        ref = oracle.flex_bwd_ref(dO64[b:b + 1, :, :q], *args, **okw)
+        for g, r, name in ((dQ[b:b + 1, :, :q], ref[0], "dQ"), (dK[b:b + 1, :, :k], ref[1], "dK"), (dV[b:b + 1, :, :k], ref[2], "dV")):
+            check(g, r, "f32", f"{name} of length {k}")
