@@ -58,6 +58,35 @@ def test_softmax_not_finite(tylo, M, dt):
     assert float((Y[6:].double() - ref).abs().max()) <= tol
 
 
+def test_softmax_row_beyond_int_packets(tylo):
+    """One row of 2^31 packets: forward at a length that is no whole number of them, backward at one that is."""
+    torch.cuda.empty_cache()
+    if torch.cuda.mem_get_info()[0] < 115e9:
+        pytest.skip("needs 105 GB")
+    M = 2 ** 33
+    buf = torch.empty(3, M + 4, device="cuda")
+    at = torch.tensor([5, 2 ** 32 + 1, M - 1, M + 2], device="cuda")
+    x = torch.tensor([0.0, 1.0, 2.0, 0.5], device="cuda")
+    X, Y = buf[0, :M + 3].view(1, -1), buf[1, :M + 3].view(1, -1)
+    X.fill_(float("-inf"))
+    X[0, at] = x
+    Y.fill_(7.0)
+    tylo.softmax_(Y, X)
+    assert torch.allclose(Y[0, at], x.softmax(0), rtol=1e-6, atol=0)
+    Y[0, at] = 0.0
+    assert not Y.any()
+    Y, dY, dX = buf[0, :M].view(1, -1), buf[1, :M].view(1, -1), buf[2, :M].view(1, -1)
+    at, y, g = at[:3], torch.tensor([0.25, 0.5, 0.25], device="cuda"), torch.tensor([1.0, 2.0, -3.0], device="cuda")
+    Y.zero_(); dY.fill_(1.0); dX.fill_(7.0)
+    Y[0, at], dY[0, at] = y, g
+    tylo.grad_softmax_(tylo.Duplicated(Y, dY), tylo.Duplicated(dX, dX))
+    assert torch.allclose(dX[0, at], y * (g - (y * g).sum()), rtol=1e-6, atol=0)
+    dX[0, at] = 0.0
+    assert not dX.any()
+    del buf, X, Y, dY, dX
+    torch.cuda.empty_cache()
+
+
 # packets per row (f32: 4 elements, 16-bit: 8): one warp, a warp and one, eight rows per CTA, ragged thread counts, 1,024 and
 # beyond (two and four packets per thread), and lengths that are not a multiple of the packet
 @pytest.mark.parametrize("dt", ["f32", "bf16"])

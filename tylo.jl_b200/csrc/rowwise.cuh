@@ -1,10 +1,9 @@
 // Row-resident building block for the bandwidth kernels (softmax, RMSNorm, LayerNorm).
 //
-// One CTA owns one row (one Julia column: the contiguous, reduced dimension of length M).
-// The row is read from HBM exactly once as 16-byte packets that stay in registers, the
-// statistics are reduced with warp shuffles plus one shared-memory hop, and the result is
-// written once.  THREADS x ITERS packets of 16 bytes cover the row; packets past the end
-// are predicated off.
+// A row is one Julia column: the contiguous, reduced dimension of length M.  THREADS threads own a row: a CTA, or a warp,
+// eight of which share a CTA.  The row is read from HBM exactly once as 16-byte packets that stay in registers, the
+// statistics are reduced with warp shuffles plus one shared-memory hop (none within a warp), and the result is written once.
+// THREADS x ITERS packets of 16 bytes cover the row; packets past the end are predicated off.
 #pragma once
 #include "common.cuh"
 
@@ -14,38 +13,43 @@ namespace tylo {
 // start at every element offset).  Packets are counted from the aligned address at or before the row's start; all but the
 // first and the last are whole and move as 16 bytes, those two element by element, so nothing outside the row is touched.
 // Every array of a call is aligned alike, so one row has the same offset in all of them.
+// Packets are counted in 64 bits: the two-pass kernels take rows as long as memory allows.
 template <typename T> struct RaggedRow {
   static constexpr int kVec = Elem<T>::kVec;
-  T* row;
+  T* base;                 // the aligned address at or before the row's start
   int off;                 // elements of packet 0 that lie before the row
-  int64_t M;
-  int nvec;
+  int64_t end;             // elements from `base` to the row's end
   __device__ __forceinline__ RaggedRow(const T* r, int64_t m)
-      : row(const_cast<T*>(r)), off((int)((reinterpret_cast<uintptr_t>(r) & 15) / sizeof(T))), M(m), nvec((int)((off + m + kVec - 1) / kVec)) {}
-  __device__ __forceinline__ bool whole(int v) const { return (v > 0 || off == 0) && (int64_t)(v + 1) * kVec <= off + M; }
+      : base(reinterpret_cast<T*>(reinterpret_cast<uintptr_t>(r) & ~uintptr_t(15))),
+        off((int)((reinterpret_cast<uintptr_t>(r) & 15) / sizeof(T))), end(off + m) {}
+  __device__ __forceinline__ int64_t nvec() const { return (end + kVec - 1) / kVec; }
+  // elements of packet v inside the row: [first, last)
+  __device__ __forceinline__ int first(int64_t v) const { return v == 0 ? off : 0; }
+  __device__ __forceinline__ int last(int64_t v) const {
+    const int64_t n = end - v * kVec;
+    return n >= kVec ? kVec : (n > 0 ? (int)n : 0);
+  }
   // packet v, elements outside the row (and packets past it) read as `fill`
-  __device__ __forceinline__ Pack<T> load(int v, float fill) const {
+  __device__ __forceinline__ Pack<T> load(int64_t v, float fill) const {
     Pack<T> p;
-    if (v < nvec && whole(v)) { p.raw = ld_stream(row - off + (size_t)v * kVec); return p; }
+    const int lo = first(v), hi = last(v);
+    const T* q = base + v * kVec;
+    if (lo == 0 && hi == kVec) { p.raw = ld_stream(q); return p; }
     float f[kVec];
 #pragma unroll
-    for (int j = 0; j < kVec; ++j) {
-      const int64_t i = (int64_t)v * kVec + j - off;
-      f[j] = (i >= 0 && i < M) ? Elem<T>::to_f(row[i]) : fill;
-    }
+    for (int j = 0; j < kVec; ++j) f[j] = j >= lo && j < hi ? Elem<T>::to_f(q[j]) : fill;
     p.pack(f);
     return p;
   }
-  __device__ __forceinline__ void store(int v, const Pack<T>& p) const {
-    if (v >= nvec) return;
-    if (whole(v)) { st_stream(row - off + (size_t)v * kVec, p.raw); return; }
+  __device__ __forceinline__ void store(int64_t v, const Pack<T>& p) const {
+    const int lo = first(v), hi = last(v);
+    T* q = base + v * kVec;
+    if (lo == 0 && hi == kVec) { st_stream(q, p.raw); return; }
     float f[kVec];
     p.unpack(f);
 #pragma unroll
-    for (int j = 0; j < kVec; ++j) {
-      const int64_t i = (int64_t)v * kVec + j - off;
-      if (i >= 0 && i < M) row[i] = Elem<T>::from_f(f[j]);
-    }
+    for (int j = 0; j < kVec; ++j)
+      if (j >= lo && j < hi) q[j] = Elem<T>::from_f(f[j]);
   }
 };
 

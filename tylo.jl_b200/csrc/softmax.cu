@@ -58,7 +58,7 @@ softmax_fwd_kernel(T* __restrict__ Y, const T* __restrict__ X, int64_t M, int N)
   RowRegs<T, THREADS, ITERS> r;
   if constexpr (RAGGED) {
     const RaggedRow<T> x(X + row * M, M);
-    nvec = (int)x.nvec;
+    nvec = (int)x.nvec();
     r.load(x, -INFINITY);
   } else {
     r.load(X + row * M, nvec);
@@ -117,7 +117,7 @@ softmax_fwd_packed_kernel(T* __restrict__ Y, const T* __restrict__ X, int64_t M,
   const size_t row = row_index<THREADS>();
   if (THREADS == 32 && row >= (size_t)N) return;
   const int tid = row_thread<THREADS>();
-  const int nvec = RAGGED ? RaggedRow<T>(X + row * M, M).nvec : (int)(M / VEC);
+  const int nvec = RAGGED ? (int)RaggedRow<T>(X + row * M, M).nvec() : (int)(M / VEC);
   RowRegs<T, THREADS, ITERS> r;
   if constexpr (RAGGED) r.load(RaggedRow<T>(X + row * M, M), -INFINITY);
   else r.load(X + row * M, nvec);
@@ -163,9 +163,9 @@ softmax_fwd_twopass_kernel(T* __restrict__ Y, const T* __restrict__ X, int64_t M
   __shared__ float smem[64];
   const size_t base = (size_t)blockIdx.x * M;
   const RaggedRow<T> x(X + base, M), y(Y + base, M);
-  const int nvec = RAGGED ? x.nvec : (int)(M / VEC);
+  const int64_t nvec = RAGGED ? x.nvec() : M / VEC;
   auto ex2 = [](float v) { return sizeof(T) == 2 ? ex2_fast(v) : exp2f(v); };
-  auto load = [&](int v) {
+  auto load = [&](int64_t v) {
     Pack<T> p;
     if constexpr (RAGGED) return x.load(v, -INFINITY);
     if (v < nvec) { p.raw = __ldg(reinterpret_cast<const uint4*>(X + base) + v); return p; }
@@ -176,7 +176,7 @@ softmax_fwd_twopass_kernel(T* __restrict__ Y, const T* __restrict__ X, int64_t M
     return p;
   };
   float m = -INFINITY, s = 0.f;
-  for (int v0 = threadIdx.x; v0 < nvec; v0 += U * THREADS) {
+  for (int64_t v0 = threadIdx.x; v0 < nvec; v0 += U * THREADS) {
     Pack<T> p[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) p[u] = load(v0 + u * THREADS);
@@ -202,13 +202,13 @@ softmax_fwd_twopass_kernel(T* __restrict__ Y, const T* __restrict__ X, int64_t M
   }
   reduce_max_sum<THREADS>(m, s, smem);
   const float inv = s == 0.f ? 0.f : 1.f / s, mo = m == -INFINITY ? 0.f : m;
-  for (int v0 = threadIdx.x; v0 < nvec; v0 += U * THREADS) {
+  for (int64_t v0 = threadIdx.x; v0 < nvec; v0 += U * THREADS) {
     Pack<T> p[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) p[u] = load(v0 + u * THREADS);
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int v = v0 + u * THREADS;
+      const int64_t v = v0 + u * THREADS;
       float f[VEC]; p[u].unpack(f);
 #pragma unroll
       for (int j = 0; j < VEC; ++j) f[j] = ex2((f[j] - mo) * kLog2e) * inv;
@@ -268,15 +268,15 @@ softmax_bwd_twopass_kernel(T* __restrict__ dX, const T* __restrict__ dY, const T
   __shared__ float smem[32];
   const size_t base = (size_t)blockIdx.x * M;
   const RaggedRow<T> ry(Y + base, M), rd(dY + base, M), ro(dX + base, M);
-  const int nvec = RAGGED ? ry.nvec : (int)(M / VEC);
-  auto load = [&](const T* p, const RaggedRow<T>& r, int v) {
+  const int64_t nvec = RAGGED ? ry.nvec() : M / VEC;
+  auto load = [&](const T* p, const RaggedRow<T>& r, int64_t v) {
     Pack<T> k;
     if constexpr (RAGGED) return r.load(v, 0.f);
     k.raw = v < nvec ? __ldg(reinterpret_cast<const uint4*>(p + base) + v) : make_uint4(0, 0, 0, 0);
     return k;
   };
   float dot = 0.f;
-  for (int v0 = threadIdx.x; v0 < nvec; v0 += U * THREADS) {
+  for (int64_t v0 = threadIdx.x; v0 < nvec; v0 += U * THREADS) {
     Pack<T> y[U], d[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) { y[u] = load(Y, ry, v0 + u * THREADS); d[u] = load(dY, rd, v0 + u * THREADS); }
@@ -289,13 +289,13 @@ softmax_bwd_twopass_kernel(T* __restrict__ dX, const T* __restrict__ dY, const T
     }
   }
   dot = block_reduce<THREADS>(dot, SumOp(), 0.f, smem);
-  for (int v0 = threadIdx.x; v0 < nvec; v0 += U * THREADS) {
+  for (int64_t v0 = threadIdx.x; v0 < nvec; v0 += U * THREADS) {
     Pack<T> y[U], d[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) { y[u] = load(Y, ry, v0 + u * THREADS); d[u] = load(dY, rd, v0 + u * THREADS); }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int v = v0 + u * THREADS;
+      const int64_t v = v0 + u * THREADS;
       float a[VEC], b[VEC];
       y[u].unpack(a); d[u].unpack(b);
 #pragma unroll
