@@ -353,25 +353,30 @@ norm_bwd_stream_kernel(T* __restrict__ dX, float* __restrict__ dWp, float* __res
 constexpr int kMaxSmem = 220 * 1024;    // dynamic shared memory asked for at most
 constexpr int kNormRowGroups = 15;      // named barriers 1..15
 
-template <typename T, bool LAYER, bool FULL>      // FULL: every thread of a row holds a packet
-__global__ void __launch_bounds__(1024)
+//
+// TPR: a thread count known to the compiler, one row per CTA; 0: tpr and R of the launch, which costs registers (in 16 bits the 64
+// of a 1,024-thread CTA do not hold the row loop without spills).  FULL: every thread of a row holds a packet.
+template <typename T, int TPR, bool LAYER, bool FULL>
+__global__ void __launch_bounds__(TPR ? TPR : 1024, TPR == 512 || (TPR && sizeof(T) == 4) ? 2 : 1)
 norm_bwd_kernel(T* __restrict__ dX, float* __restrict__ dWp, float* __restrict__ dBp, const T* __restrict__ dY,
                 const T* __restrict__ X, const T* __restrict__ W, const float* __restrict__ Mean,
-                const float* __restrict__ Rstd, int M, int N, float offset, int tpr, int R) {
+                const float* __restrict__ Rstd, int M, int N, float offset, int tpr_, int R_) {
   constexpr int VEC = Elem<T>::kVec;
   extern __shared__ __align__(16) float sm[];
+  const int tpr = TPR ? TPR : tpr_, R = TPR ? 1 : R_;
   const int nvec = FULL ? tpr : M / VEC, wpr = tpr >> 5;
-  const int rg = threadIdx.x / tpr, v = threadIdx.x % tpr, lane = threadIdx.x & 31, wr = v >> 5;
+  const int rg = TPR ? 0 : threadIdx.x / tpr, v = TPR ? threadIdx.x : threadIdx.x % tpr, lane = threadIdx.x & 31, wr = v >> 5;
   float* red = sm + rg * 2 * 64;               // [parity][64]
   float* tot = sm + R * 2 * 64;                // the CTA's dW (and dB) partials, R > 1
+  // threads past the row's end read its last packet (no branch around the loads) and take no part in the sums and stores
   const bool live = FULL || v < nvec;
-  const int col = v * VEC;
+  const int col = (live ? v : nvec - 1) * VEC;
   const float inv_m = 1.0f / (float)M;
   float g[VEC], dw[VEC], db[VEC];
-  if (live) ld_param(W + col).unpack(g);
+  ld_param(W + col).unpack(g);
 #pragma unroll
   for (int j = 0; j < VEC; ++j) {
-    g[j] = live ? (LAYER ? g[j] : g[j] + offset) : 0.f;
+    if constexpr (!LAYER) g[j] += offset;
     dw[j] = 0.f; db[j] = 0.f;
   }
   // rows are counted in unsigned: N may be 2^31 - 1, and the row asked for ahead lies up to 2 x 296 x 15 beyond (see the launch)
@@ -381,23 +386,24 @@ norm_bwd_kernel(T* __restrict__ dX, float* __restrict__ dWp, float* __restrict__
   float r0 = 0.f, r1 = 0.f, r2 = 0.f, m0 = 0.f, m1 = 0.f, m2 = 0.f;
   auto fetch = [&](unsigned r, Pack<T>& x, Pack<T>& d, float& rs, float& mn) {
     if (r < rows) {
-      if (live) { x.raw = ld_stream(X + (size_t)r * M + col); d.raw = ld_stream(dY + (size_t)r * M + col); }
+      x.raw = ld_stream(X + (size_t)r * M + col); d.raw = ld_stream(dY + (size_t)r * M + col);
       rs = Rstd[r];
       mn = LAYER ? Mean[r] : 0.f;
     }
   };
-  // rows in flight behind the current one: two for RMSNorm, one for LayerNorm (its extra accumulators
-  // and statistics would otherwise push the 1024-thread CTA past 64 registers per thread)
+  // rows in flight behind the current one: two for RMSNorm; one for LayerNorm (its extra accumulators and statistics would push
+  // the 1024-thread CTA past 64 registers per thread) and in 16 bits with launch-time counts (rms bf16 512: 180 us with two, 144)
+  constexpr bool kTwo = !LAYER && (TPR || VEC == 4);
   unsigned row = blockIdx.x * (unsigned)R + rg;
   fetch(row, x0, d0, r0, m0);
-  if constexpr (!LAYER) fetch(row + stride, x1, d1, r1, m1);
+  if constexpr (kTwo) fetch(row + stride, x1, d1, r1, m1);
   for (int par = 0; row < rows; row += stride, par ^= 1) {
-    if constexpr (LAYER) fetch(row + stride, x1, d1, r1, m1);
+    if constexpr (!kTwo) fetch(row + stride, x1, d1, r1, m1);
     else fetch(row + 2 * stride, x2, d2, r2, m2);
     float s1 = 0.f, s2 = 0.f;
     const uint64_t nm2 = sm100::pack_f32x2(-m0, -m0), r2p = sm100::pack_f32x2(r0, r0);
     {
-      // packed fp32 pairs: xhat = (x - mean) rstd, gd = g dy, s1 += xhat gd, s2 += gd  (dead lanes have g = 0)
+      // packed fp32 pairs: xhat = (x - mean) rstd, gd = g dy, s1 += xhat gd, s2 += gd
       float xf[VEC], df[VEC];
       x0.unpack(xf); d0.unpack(df);
       uint64_t a1 = 0ull, a2 = 0ull;
@@ -411,13 +417,15 @@ norm_bwd_kernel(T* __restrict__ dX, float* __restrict__ dWp, float* __restrict__
       float lo, hi;
       sm100::unpack_f32x2(a1, lo, hi); s1 = lo + hi;
       if constexpr (LAYER) { sm100::unpack_f32x2(a2, lo, hi); s2 = lo + hi; }
+      if (!live) { s1 = 0.f; s2 = 0.f; }
     }
     s1 = warp_reduce(s1, SumOp());
     if constexpr (LAYER) s2 = warp_reduce(s2, SumOp());
     if (wpr > 1) {
       float* rp = red + par * 64;
       if (lane == 0) { rp[wr] = s1; rp[32 + wr] = s2; }
-      asm volatile("bar.sync %0, %1;" ::"r"(rg + 1), "r"(tpr) : "memory");
+      if constexpr (TPR) __syncthreads();
+      else asm volatile("bar.sync %0, %1;" ::"r"(rg + 1), "r"(tpr) : "memory");
       s1 = warp_reduce(lane < wpr ? rp[lane] : 0.f, SumOp());
       if constexpr (LAYER) s2 = warp_reduce(lane < wpr ? rp[32 + lane] : 0.f, SumOp());
     }
@@ -446,7 +454,7 @@ norm_bwd_kernel(T* __restrict__ dX, float* __restrict__ dWp, float* __restrict__
     Pack<T> out; out.pack(o);
     if (live) st_stream(dX + (size_t)row * M + col, out.raw);
     x0 = x1; d0 = d1; r0 = r1; m0 = m1;
-    if constexpr (!LAYER) { x1 = x2; d1 = d2; r1 = r2; m1 = m2; }
+    if constexpr (kTwo) { x1 = x2; d1 = d2; r1 = r2; m1 = m2; }
   }
   // sum over the row groups, in their order
   for (int k = 1; k < R; ++k) {
@@ -703,8 +711,8 @@ static int32_t norm_bwd_launch(void* dX, void* dW, void* dB, const void* dY, con
   };
   unsigned grid;
   if (nvec == 1024 || nvec == 512) {
-    // one packet per thread and a CTA size known to the compiler: 64 registers without spills (rms 8192 bf16, 8,192 rows,
-    // forward + backward: 131 us; 164 us in the general form below)
+    // a kernel of their own for whole CTAs: 2^27 bytes of X in us, backward, here / in norm_bwd_kernel at 1,024 or 512 threads: RMS
+    // bf16 1,024 packets 152 / 160, 512 149 / 152, fp32 512 145 / 152; LayerNorm is level (172 / 172, 160 / 158)
     grid = walkers(N, nvec == 1024 ? 1 : 2);
     if (nvec == 1024)
       norm_bwd_stream_kernel<T, 1024, LAYER><<<grid, 1024, 0, st>>>(
@@ -712,6 +720,24 @@ static int32_t norm_bwd_launch(void* dX, void* dW, void* dB, const void* dY, con
     else
       norm_bwd_stream_kernel<T, 512, LAYER><<<grid, 512, 0, st>>>(
           (T*)dX, dWp, dBp, (const T*)dY, (const T*)X, (const T*)W, Mean, Rstd, (int)M, N, offset);
+  } else if (nvec > (VEC == 8 ? 256 : 512) && nvec <= (VEC == 8 ? 1024 : 768)) {
+    // thread counts known to the compiler, up to a quarter of them idle; fp32 fits two such CTAs per SM.  us, launch-time counts /
+    // these: RMS bf16 300 packets 290 / 219, 513 347 / 208, 1,000 245 / 166; LayerNorm bf16 1,000 273 / 173; fp32 RMS 513 209 / 162,
+    // 768 164 / 137 (850 at 896 threads, where only one CTA fits, 167 / 166: left on launch-time counts)
+    auto run = [&](auto kern, int threads, int per_sm) {
+      grid = walkers(N, per_sm);
+      kern<<<grid, threads, 2 * 64 * 4, st>>>((T*)dX, dWp, dBp, (const T*)dY, (const T*)X, (const T*)W, Mean, Rstd, (int)M, (int)N, offset, 0, 1);
+    };
+    if constexpr (VEC == 8) {
+      if (nvec <= 512) run(norm_bwd_kernel<T, 512, LAYER, false>, 512, 2);
+      else if (nvec <= 640) run(norm_bwd_kernel<T, 640, LAYER, false>, 640, 1);
+      else if (nvec <= 768) run(norm_bwd_kernel<T, 768, LAYER, false>, 768, 1);
+      else if (nvec <= 896) run(norm_bwd_kernel<T, 896, LAYER, false>, 896, 1);
+      else run(norm_bwd_kernel<T, 1024, LAYER, false>, 1024, 1);
+    } else {
+      if (nvec <= 640) run(norm_bwd_kernel<T, 640, LAYER, false>, 640, 2);
+      else run(norm_bwd_kernel<T, 768, LAYER, false>, 768, 2);
+    }
   } else if (nvec >= 1 && nvec <= 1024) {
     const int tpr = (int)(nvec + 31) / 32 * 32;
     // as many rows per CTA as make 512 threads, fewer when there are not enough rows to occupy every SM with that
@@ -722,7 +748,7 @@ static int32_t norm_bwd_launch(void* dX, void* dW, void* dB, const void* dY, con
     if (R < 1) R = 1;
     grid = walkers((N + R - 1) / R, tpr * R > 512 ? 1 : 2);
     const size_t smem = (size_t)R * 2 * 64 * 4 + (R > 1 ? acc_bytes : 0);
-    auto kern = nvec == tpr ? norm_bwd_kernel<T, LAYER, true> : norm_bwd_kernel<T, LAYER, false>;
+    auto kern = nvec == tpr ? norm_bwd_kernel<T, 0, LAYER, true> : norm_bwd_kernel<T, 0, LAYER, false>;
     // (several rows per CTA means rows of at most 256 packets: below the 48 KB that need no attribute)
     kern<<<grid, tpr * R, smem, st>>>((T*)dX, dWp, dBp, (const T*)dY, (const T*)X, (const T*)W, Mean, Rstd, (int)M, (int)N,
                                       offset, tpr, R);
