@@ -93,7 +93,7 @@ def test_softmax_row_beyond_int_packets(tylo):
 @pytest.mark.parametrize("M,N,groups", [(8, 40, 296), (256, 700, 296), (264, 31, 3), (520, 5000, 296), (4104, 301, 296), (8192, 3, 1),
                                         (8200, 17, 5), (12288, 200, 296), (16384, 9, 296), (16392, 3, 296), (1, 7, 296), (1001, 333, 296),
                                         (33001, 2, 296), (2056, 310, 296), (3080, 30, 296), (5128, 160, 296), (6152, 9, 7),
-                                        (7176, 5, 296)])
+                                        (7176, 5, 296), (6251, 3, 296), (7043, 300, 296), (9401, 5, 3)])
 def test_norm_rows(tylo, oracle, M, N, groups, dt):
     rng = np.random.default_rng(M + N)
     eps = 1e-5

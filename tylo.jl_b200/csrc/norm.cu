@@ -575,7 +575,7 @@ norm_bwd_wide_kernel(T* __restrict__ dX, float* __restrict__ dWp, float* __restr
   }
 }
 
-// Any M / alignment: element accesses.  While the row and the partials fit shared memory (SMEM), X and dY are read from
+// Any M / alignment: element accesses.  While the row and the partials of several CTAs fit shared memory (SMEM), X and dY are read from
 // memory once, the row waits in shared memory as fp32 and the partials are added up there; beyond that the CTA's partial row
 // is accumulated in global memory (the CTA is its only writer) and the row read twice.
 template <typename T, bool LAYER, bool SMEM>
@@ -764,10 +764,14 @@ static int32_t norm_bwd_launch(void* dX, void* dW, void* dB, const void* dY, con
     if (nvec <= 2048) TYLO_BWD_WIDE(2); else TYLO_BWD_WIDE(4);
 #undef TYLO_BWD_WIDE
   } else {
+    // through shared memory while three CTAs (RMSNorm) or two (LayerNorm, whose partials are twice the traffic in global memory) fit
+    // an SM; with fewer, the rows wait for one another longer than the second read takes.  us, shared / global memory, 2^26
+    // elements: RMSNorm bf16 7,001 elements 333 / 291, 16,383 576 / 320, fp32 9,401 723 / 375; LayerNorm bf16 7,001 (two CTAs)
+    // 342 / 415, 8,101 (one) 575 / 430.
     const int64_t smem = acc_bytes + 2 * M * 4;
-    const int per_sm = smem <= kMaxSmem / 3 ? 3 : (smem <= kMaxSmem / 2 ? 2 : 1);
-    grid = walkers(N, smem <= kMaxSmem ? per_sm : 2);
-    if (smem <= kMaxSmem) {
+    const bool in_smem = smem <= kMaxSmem / (LAYER ? 2 : 3);
+    grid = walkers(N, smem <= kMaxSmem / 3 ? 3 : 2);
+    if (in_smem) {
       auto kern = norm_bwd_generic_kernel<T, LAYER, true>;
       if (int32_t rc = allow_smem(kern, smem)) return rc;
       kern<<<grid, 512, smem, st>>>((T*)dX, dWp, dBp, (const T*)dY, (const T*)X, (const T*)W, Mean, Rstd, M, N, offset);
