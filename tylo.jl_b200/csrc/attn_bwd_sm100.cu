@@ -344,7 +344,8 @@ attn_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       // One elected lane, chosen by elect.sync: the compiler then knows that a single thread runs this branch and keeps
       // descriptors and tensor-memory addresses in uniform registers.  Behind `if (lane == 0)` every tcgen05.mma with both
       // operands in shared memory cost its issuer 118 clocks; issued like this it takes 65, the tensor pipe's own time
-      // (128 x 128 x 16).  Forward and backward of B 4, S 4096, 32 / 8 heads, D 128: 2,890 -> 2,630 us.
+      // (128 x 128 x 16).  Forward and backward of B 4, S 4096, 32 / 8 heads, D 128: 2,890 -> 2,630 us in isolated passes,
+      // 2,856 -> 2,756 back to back, where the chip is at its power cap.
       constexpr uint32_t idesc_ss = idesc_f16(Fmt<T>::v, 0, 0, BT, BT);
       constexpr uint32_t idesc_ts = idesc_f16(Fmt<T>::v, 0, 1, BT, D);
       const uint64_t dk_hi = smem_desc_sw128(0, 16, 1024);            // K-major operand

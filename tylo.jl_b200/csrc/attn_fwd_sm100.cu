@@ -132,7 +132,7 @@ __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.w
 
 // The form of the tile loop (see softmax_tile).  In the register-resident form P is handed to the MMA issuer in two parts:
 // the product over the first 96 keys runs under the exponentials of the last 32, so that only a quarter of P V is left in
-// the chain softmax -> P V -> Q K^T of a Q tile (causal forward, S 4096, D 128: 488 -> 480 us).
+// the chain softmax -> P V -> Q K^T of a Q tile (causal forward, S 4096, D 128, isolated passes: 488 -> 480 us).
 constexpr bool fwd_chunked(uint32_t mask, uint32_t score) { return (mask & ~(uint32_t)TYLO_MASK_CAUSAL) != 0 || score != 0; }
 
 struct TileRange { int s, e; };  // CTA-local key-tile indices [s, e) a Q tile takes part in
@@ -928,7 +928,8 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       // One elected lane, chosen by elect.sync: the compiler then knows that a single thread runs this branch and keeps
       // descriptors and tensor-memory addresses in uniform registers.  Behind `if (lane == 0)` every tcgen05.mma with both
       // operands in shared memory cost its issuer 118 clocks; issued like this it takes 65, the tensor pipe's own time
-      // (128 x 128 x 16).  Causal forward of B 4, S 4096, 32 / 8 heads, D 128: 550 -> 488 us.
+      // (128 x 128 x 16).  Causal forward of B 4, S 4096, 32 / 8 heads, D 128, together with P in two parts: 550 -> 480 us in
+      // isolated passes, 604 -> 566 back to back, where the chip is at its power cap.
       if (elect_one()) {
         constexpr uint32_t idesc_qk = idesc_f16(MmaFmt<T>::v, 0, 0, BM, BN);
         constexpr uint32_t idesc_pv = idesc_f16(MmaFmt<T>::v, 0, 1, BM, D);
