@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("dt", ["f32", "bf16", "f16"])
 @pytest.mark.parametrize("M,N", [(1, 5), (7, 9), (9, 3), (63, 4), (513, 3), (2049, 3), (4095, 3), (8193, 2), (65533, 2), (65544, 2),
-                                 (70001, 2), (131072, 1)])
+                                 (70001, 2), (131072, 1), (12292, 18), (33001, 30), (40000, 74), (33000, 150)])
 def test_softmax_rows(tylo, oracle, M, N, dt):
     rng = np.random.default_rng(M + N)
     buf = torch.full((N * M + 32,), 7.0, device="cuda", dtype={"f32": torch.float32, "bf16": torch.bfloat16, "f16": torch.float16}[dt])

@@ -8,7 +8,11 @@
 // exp is evaluated once per element: each thread first takes the max of its own elements,
 // exponentiates against that, and the result is rescaled by exp2(m_thread - m_row) / sum
 // — one extra exp per thread instead of one per element.
+#include <cooperative_groups.h>
+
 #include "rowwise.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace tylo {
 
@@ -156,12 +160,17 @@ softmax_fwd_packed_kernel(T* __restrict__ Y, const T* __restrict__ X, int64_t M,
 
 // Rows too long for one CTA's registers, forward: a pass that keeps a running (max, sum) per thread and a pass that reads
 // the row again out of L2 (see the backward's two-pass form below) and writes.
-template <typename T, int THREADS, bool RAGGED>
+// CLUSTERED: a row is dealt packet by packet over the CTAs of a cluster, which exchange their (max, sum) through distributed
+// shared memory; for launches with fewer rows than SMs.  Each thread reads and writes the same packets in both passes.
+template <typename T, int THREADS, bool RAGGED, bool CLUSTERED>
 __global__ void __launch_bounds__(THREADS)
 softmax_fwd_twopass_kernel(T* __restrict__ Y, const T* __restrict__ X, int64_t M) {
   constexpr int VEC = Elem<T>::kVec, U = 4;
-  __shared__ float smem[64];
-  const size_t base = (size_t)blockIdx.x * M;
+  __shared__ float smem[66];
+  int ctas = 1, rank = 0;
+  if constexpr (CLUSTERED) { ctas = cg::this_cluster().num_blocks(); rank = cg::this_cluster().block_rank(); }
+  const int step = ctas * THREADS, first = rank * THREADS + (int)threadIdx.x;
+  const size_t base = (size_t)(blockIdx.x / ctas) * M;
   const RaggedRow<T> x(X + base, M), y(Y + base, M);
   const int64_t nvec = RAGGED ? x.nvec() : M / VEC;
   auto ex2 = [](float v) { return sizeof(T) == 2 ? ex2_fast(v) : exp2f(v); };
@@ -176,10 +185,10 @@ softmax_fwd_twopass_kernel(T* __restrict__ Y, const T* __restrict__ X, int64_t M
     return p;
   };
   float m = -INFINITY, s = 0.f;
-  for (int64_t v0 = threadIdx.x; v0 < nvec; v0 += U * THREADS) {
+  for (int64_t v0 = first; v0 < nvec; v0 += U * step) {
     Pack<T> p[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) p[u] = load(v0 + u * THREADS);
+    for (int u = 0; u < U; ++u) p[u] = load(v0 + u * step);
     float mx = -INFINITY;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -201,14 +210,25 @@ softmax_fwd_twopass_kernel(T* __restrict__ Y, const T* __restrict__ X, int64_t M
     }
   }
   reduce_max_sum<THREADS>(m, s, smem);
+  if constexpr (CLUSTERED) {
+    cg::cluster_group cluster = cg::this_cluster();
+    if (threadIdx.x == 0) { smem[64] = m; smem[65] = s; }
+    cluster.sync();
+    const int lane = threadIdx.x & 31;
+    const float* peer = cluster.map_shared_rank(smem, lane < ctas ? lane : 0);
+    m = lane < ctas ? peer[64] : -INFINITY;
+    s = lane < ctas ? peer[65] : 0.f;
+    reduce_max_sum<32>(m, s, smem);
+    cluster.sync();               // a CTA may leave, and take its shared memory along, once everyone has read it
+  }
   const float inv = s == 0.f ? 0.f : 1.f / s, mo = m == -INFINITY ? 0.f : m;
-  for (int64_t v0 = threadIdx.x; v0 < nvec; v0 += U * THREADS) {
+  for (int64_t v0 = first; v0 < nvec; v0 += U * step) {
     Pack<T> p[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) p[u] = load(v0 + u * THREADS);
+    for (int u = 0; u < U; ++u) p[u] = load(v0 + u * step);
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int64_t v = v0 + u * THREADS;
+      const int64_t v = v0 + u * step;
       float f[VEC]; p[u].unpack(f);
 #pragma unroll
       for (int j = 0; j < VEC; ++j) f[j] = ex2((f[j] - mo) * kLog2e) * inv;
@@ -337,7 +357,24 @@ static int32_t softmax_launch(void* out, const void* a, const void* b, int64_t M
 #undef TYLO_SM_LAUNCH
   // rows too long for one CTA's registers: the two-pass form (backward of 4096 x 32768 bf16: 4,952 GB/s with a clustered
   // register-resident form, 6,225 with this one at 1,024 threads; 5,317 at 512 and 4,042 at 256 threads)
-  if constexpr (FWD) softmax_fwd_twopass_kernel<T, 1024, RAGGED><<<(unsigned)N, 1024, 0, st>>>((T*)out, (const T*)a, M);
+  if constexpr (FWD) {
+    // more than 8,192 packets and fewer rows than SMs: each over the largest cluster of 8, 4 or 2 CTAs that leaves an SM per CTA.
+    // fp32, cold, us, one CTA / cluster: 65,536 elements x 1 row 18.4 / 12.3, x 64 18.4 / 16.3; 131,072 x 1 28.7 / 12.3, x 64
+    // 30.7 / 24.6; 2^20 x 1 166 / 31.  At 3,072 and 4,096 packets the cluster's two barriers cost more than they save (10.2 / 12.3).
+    unsigned c = nvec > 8192 ? 8 : 1;
+    while (c > 1 && c * N > sm_count()) c /= 2;
+    if (c > 1) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3((unsigned)N * c); cfg.blockDim = dim3(1024); cfg.stream = st;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = c; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr; cfg.numAttrs = 1;
+      TYLO_CUDA_OK(cudaLaunchKernelEx(&cfg, softmax_fwd_twopass_kernel<T, 1024, RAGGED, true>, (T*)out, (const T*)a, M));
+      return TYLO_OK;
+    }
+    softmax_fwd_twopass_kernel<T, 1024, RAGGED, false><<<(unsigned)N, 1024, 0, st>>>((T*)out, (const T*)a, M);
+  }
   else softmax_bwd_twopass_kernel<T, 1024, RAGGED><<<(unsigned)N, 1024, 0, st>>>((T*)out, (const T*)a, (const T*)b, M);
   return check_launch(what);
 }
