@@ -358,11 +358,12 @@ static int32_t softmax_launch(void* out, const void* a, const void* b, int64_t M
   // rows too long for one CTA's registers: the two-pass form (backward of 4096 x 32768 bf16: 4,952 GB/s with a clustered
   // register-resident form, 6,225 with this one at 1,024 threads; 5,317 at 512 and 4,042 at 256 threads)
   if constexpr (FWD) {
-    // more than 8,192 packets and fewer rows than SMs: each over the largest cluster of 8, 4 or 2 CTAs that leaves an SM per CTA.
+    // more than 8,192 packets and fewer rows than SMs: each over the largest cluster of 8, 4 or 2 CTAs that leaves an SM per CTA, an
+    // eighth of the SMs kept back (clusters do not span the chip's processor groups: 18 clusters of 8 took two waves, 22.5 us for 14.3).
     // fp32, cold, us, one CTA / cluster: 65,536 elements x 1 row 18.4 / 12.3, x 64 18.4 / 16.3; 131,072 x 1 28.7 / 12.3, x 64
     // 30.7 / 24.6; 2^20 x 1 166 / 31.  At 3,072 and 4,096 packets the cluster's two barriers cost more than they save (10.2 / 12.3).
     unsigned c = nvec > 8192 ? 8 : 1;
-    while (c > 1 && c * N > sm_count()) c /= 2;
+    while (c > 1 && 8 * c * N > 7 * sm_count()) c /= 2;
     if (c > 1) {
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3((unsigned)N * c); cfg.blockDim = dim3(1024); cfg.stream = st;
