@@ -162,7 +162,8 @@ softmax_fwd_packed_kernel(T* __restrict__ Y, const T* __restrict__ X, int64_t M,
 // the row again out of L2 (see the backward's two-pass form below) and writes.
 // CLUSTERED: a row is dealt packet by packet over the CTAs of a cluster, which exchange their (max, sum) through distributed
 // shared memory; for launches with fewer rows than SMs.  Each thread reads and writes the same packets in both passes.
-template <typename T, int THREADS, bool RAGGED, bool CLUSTERED>
+// ONCE: the row is no longer than U packets per thread, which wait in registers for the second pass.
+template <typename T, int THREADS, bool RAGGED, bool CLUSTERED, bool ONCE>
 __global__ void __launch_bounds__(THREADS)
 softmax_fwd_twopass_kernel(T* __restrict__ Y, const T* __restrict__ X, int64_t M) {
   constexpr int VEC = Elem<T>::kVec, U = 4;
@@ -185,8 +186,8 @@ softmax_fwd_twopass_kernel(T* __restrict__ Y, const T* __restrict__ X, int64_t M
     return p;
   };
   float m = -INFINITY, s = 0.f;
+  Pack<T> p[U];
   for (int64_t v0 = first; v0 < nvec; v0 += U * step) {
-    Pack<T> p[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) p[u] = load(v0 + u * step);
     float mx = -INFINITY;
@@ -223,9 +224,10 @@ softmax_fwd_twopass_kernel(T* __restrict__ Y, const T* __restrict__ X, int64_t M
   }
   const float inv = s == 0.f ? 0.f : 1.f / s, mo = m == -INFINITY ? 0.f : m;
   for (int64_t v0 = first; v0 < nvec; v0 += U * step) {
-    Pack<T> p[U];
+    if constexpr (!ONCE) {
 #pragma unroll
-    for (int u = 0; u < U; ++u) p[u] = load(v0 + u * step);
+      for (int u = 0; u < U; ++u) p[u] = load(v0 + u * step);
+    }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int64_t v = v0 + u * step;
@@ -362,19 +364,25 @@ static int32_t softmax_launch(void* out, const void* a, const void* b, int64_t M
     // eighth of the SMs kept back (clusters do not span the chip's processor groups: 18 clusters of 8 took two waves, 22.5 us for 14.3).
     // fp32, cold, us, one CTA / cluster: 65,536 elements x 1 row 18.4 / 12.3, x 64 18.4 / 16.3; 131,072 x 1 28.7 / 12.3, x 64
     // 30.7 / 24.6; 2^20 x 1 166 / 31.  At 3,072 and 4,096 packets the cluster's two barriers cost more than they save (10.2 / 12.3).
-    unsigned c = nvec > 8192 ? 8 : 1;
-    while (c > 1 && 8 * c * N > 7 * sm_count()) c /= 2;
-    if (c > 1) {
+    // Up to 8,192 packets and a quarter as many rows as SMs: clusters of 4 or 8 CTAs of 256 threads that hold the row in registers.
+    // us back to back, one CTA / cluster: fp32 16,384 elements x 1 row 5.2 / 4.6, 32,768 x 1 7.1 / 4.7, x 32 7.2 / 6.6; bf16 65,536 x 1
+    // 8.8 / 4.7, x 37 9.0 / 7.2.
+    auto clusters = [&](auto kern, unsigned c, unsigned threads) -> int32_t {
       cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3((unsigned)N * c); cfg.blockDim = dim3(1024); cfg.stream = st;
+      cfg.gridDim = dim3((unsigned)N * c); cfg.blockDim = dim3(threads); cfg.stream = st;
       cudaLaunchAttribute attr[1];
       attr[0].id = cudaLaunchAttributeClusterDimension;
       attr[0].val.clusterDim.x = c; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
       cfg.attrs = attr; cfg.numAttrs = 1;
-      TYLO_CUDA_OK(cudaLaunchKernelEx(&cfg, softmax_fwd_twopass_kernel<T, 1024, RAGGED, true>, (T*)out, (const T*)a, M));
+      TYLO_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, (T*)out, (const T*)a, M));
       return TYLO_OK;
-    }
-    softmax_fwd_twopass_kernel<T, 1024, RAGGED, false><<<(unsigned)N, 1024, 0, st>>>((T*)out, (const T*)a, M);
+    };
+    if (nvec <= 8192 && N <= sm_count() / 4)
+      return clusters(softmax_fwd_twopass_kernel<T, 256, RAGGED, true, true>, nvec <= 4096 ? 4 : 8, 256);
+    unsigned c = nvec > 8192 ? 8 : 1;
+    while (c > 1 && 8 * c * N > 7 * sm_count()) c /= 2;
+    if (c > 1) return clusters(softmax_fwd_twopass_kernel<T, 1024, RAGGED, true, false>, c, 1024);
+    softmax_fwd_twopass_kernel<T, 1024, RAGGED, false, false><<<(unsigned)N, 1024, 0, st>>>((T*)out, (const T*)a, M);
   }
   else softmax_bwd_twopass_kernel<T, 1024, RAGGED><<<(unsigned)N, 1024, 0, st>>>((T*)out, (const T*)a, (const T*)b, M);
   return check_launch(what);
